@@ -55,32 +55,15 @@ bool smooth(int n)
     return n == 1;
 }
 
-// Radix schedule: radix 16 first, then 8, 4, 2 and the odd radices (256 is
-// two radix-16 stages: one shared-memory exchange per transform).
+// Radix schedule (radix_seq, shared with the compiled transforms and the
+// shared-memory sizes derived from them).
 bool make_plan(int n, FftPlan* p)
 {
+    const RadixSeq q = radix_seq(n);
     p->n = n;
-    p->nst = 0;
-    int m = n;
-    while (m % 16 == 0 && p->nst < kMaxStages) { p->rad[p->nst++] = 16; m /= 16; }
-    while (m % 8 == 0 && p->nst < kMaxStages) { p->rad[p->nst++] = 8; m /= 8; }
-    while (m % 4 == 0 && p->nst < kMaxStages) { p->rad[p->nst++] = 4; m /= 4; }
-    while (m % 2 == 0 && p->nst < kMaxStages) { p->rad[p->nst++] = 2; m /= 2; }
-    for (int r : {3, 5, 7})
-        while (m % r == 0 && p->nst < kMaxStages) { p->rad[p->nst++] = r; m /= r; }
-    if (m != 1) return false;
-    if (p->nst == 1 && p->rad[0] == 16) {  // n = 16: two radix-4 stages
-        p->rad[0] = 4;
-        p->rad[1] = 4;
-        p->nst = 2;
-    }
-    if (p->nst < 2) return false;
-    // the compile-time transforms (and the shared-memory sizes derived from
-    // them) use the same radix sequence
-    if (p->nst != ct_nst(n)) return false;
-    for (int st = 0; st < p->nst; ++st)
-        if (p->rad[st] != ct_rad(n, st)) return false;
-    return true;
+    p->nst = q.nst;
+    for (int s = 0; s < kMaxStages; ++s) p->rad[s] = q.rad[s];
+    return q.nst >= 2;
 }
 
 // FP64 construction of the 1D tables of one axis on the GPU:

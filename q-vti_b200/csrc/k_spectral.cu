@@ -1,0 +1,287 @@
+// Spectral passes of the time step: z transforms of the velocities, y lines,
+// and the k-space x pass with the constant-Q operators.
+#include "step_common.cuh"
+
+namespace qvti {
+
+namespace {
+
+// Derivative bookkeeping for the 9 stress-side derivatives d (G index
+// o = 3 d + j): component, axis, forward(1)/backward(0) staggered shift.
+// d: 0 dx vx, 1 dy vy, 2 dz vz (forward shift, kvx_x kvy_y kvz_z),
+//    3 dz vx, 4 dx vz, 5 dy vx, 6 dx vy, 7 dz vy, 8 dy vz (backward shift)
+// -- the table assignment of cuviscoelas_3D.cu:1342-1562.
+__constant__ int c_comp[9] = {0, 1, 2, 0, 2, 0, 1, 1, 2};
+__constant__ int c_axis[9] = {0, 1, 2, 2, 0, 1, 0, 2, 1};
+__constant__ int c_fwd[9] = {1, 1, 1, 0, 0, 0, 0, 0, 0};
+// G indices that go through the x and y passes (all but kGz)
+__constant__ int c_gxy[kNumGxy] = {0, 1, 2, 3, 5, 6, 8, 9, 11, 12, 13, 14, 15, 17, 18, 19, 20, 21, 23, 24, 26};
+
+// ------------------------------------------------------------------ k_fz --
+// R2C along z of vx, vy, vz.  Tile: one x, P consecutive y rows (P even);
+// rows (2q, 2q+1) share one complex transform.  Output H[f][kz][x][y].
+template <int N>
+__global__ void __launch_bounds__(kThreads) k_fz(KP k, int P_rt)
+{
+    extern __shared__ float4 smem4[];
+    float2* sm = reinterpret_cast<float2*>(smem4);
+    const int P = N > 0 ? 16 : P_rt;
+    const int n = N > 0 ? N : k.nz, Qp = P / 2, ps = n + n / 16;
+    float2* tw = sm;
+    float2* A = tw + n;
+    float2* B = A + Qp * ps;
+    load_table(tw, k.tw_z, n);
+    __syncthreads();
+    const int f = blockIdx.z, x = blockIdx.y, y0 = blockIdx.x * P;
+    const int yv = min(P, k.ny - y0);  // rows of the tile inside the grid (even)
+    const float* src = k.v[f];
+    float2* Z = out_any<N, 8, kThreads, kLinePad>(k.pz, A, B);
+    auto load = [&](int q, int i) -> float2 {
+        if (2 * q >= yv) return make_float2(0.f, 0.f);
+        const int b = cell(k, x, y0 + 2 * q, i);
+        return make_float2(src[b], src[b + n]);
+    };
+    auto store = [&](int q, int i, float2 v) { Z[q * ps + i] = v; };
+    fft_any<N, 8, kThreads, kLinePad, false>(k.pz, tw, A, B, Qp, ps, 1, load, store);
+    float2* H = k.H[f];
+    for (int t = threadIdx.x; t < k.nkz * P; t += blockDim.x) {
+        const int p = t % P, kz = t / P, q = p >> 1;
+        if (p >= yv) continue;
+        const float2 z = Z[q * ps + kz];
+        const float2 zm = cconj(Z[q * ps + (kz ? n - kz : 0)]);
+        H[spec(k, kz, x, y0 + p)] = (p & 1) ? unpack_b(z, zm) : unpack_a(z, zm);
+    }
+}
+
+// ------------------------------------------------------------------ k_cy --
+// C2C along y, in place, on L contiguous y lines per block (lines (kz, x)
+// starting at line0).  Line-major mapping on a padded tile: each half warp
+// reads or writes 16 consecutive points (128 bytes) of one line, so a warp
+// access touches two lines, and the radix-16 shared-memory stages are
+// conflict-free.  The field is H[0..2] (forward) or G[0..26] (inverse), by
+// blockIdx.y.
+constexpr int kCyThreads = 128;  // L = 8 lines x 256 points = one radix-16 butterfly per thread
+
+template <int N, bool INV>
+__global__ void __launch_bounds__(kCyThreads) k_cy(KP k, int L_rt, long long line0, long long line_end)
+{
+    extern __shared__ float4 smem4[];
+    float2* sm = reinterpret_cast<float2*>(smem4);
+    const int L = N > 0 ? 8 : L_rt;
+    const int n = N > 0 ? N : k.ny;
+    float2* tw = sm;
+    float2* A = tw + n;
+    float2* B = A + L * (n + n / 16);
+    float2* C = B + L * (n + n / 16);  // forward with Yv: the lines' y spectra, [L][n]
+    load_table(tw, k.tw_y, n);
+    __syncthreads();
+    // forward: H -> Hy (H stays for k_sigma's kz-only fields); inverse: G in
+    // place, blockIdx.y over the fields that went through k_mx
+    const int c = blockIdx.y;
+    const long long first = line0 + (long long)blockIdx.x * L;
+    const int lv = (int)min((long long)L, line_end - first);  // lines of the tile inside the batch
+    const long long off = first * n;
+    const float2* src = (INV ? k.G[c_gxy[c]] : k.H[c]) + off;
+    float2* dst = (INV ? k.G[c_gxy[c]] : k.Hy[c]) + off;
+    const bool ydv = !INV && k.Yv[c] != nullptr;
+    auto load = [&](int p, int i) -> float2 { return p < lv ? src[(long long)p * n + i] : make_float2(0.f, 0.f); };
+    auto store = [&](int p, int i, float2 v) {
+        if (p < lv) dst[(long long)p * n + i] = v;
+        if (ydv) C[p * n + i] = v;
+    };
+    fft_any<N, 8, kCyThreads, kLinePad, INV>(k.py, tw, A, B, L, n + n / 16, 1, load, store);
+    if constexpr (!INV) {
+        if (ydv) {
+            // the y derivative with the identity dispersion operator, scaled
+            // by 1/(ny nz) like a field of the x and y passes (1/ntp times
+            // the x round trip's nx): dy vy (c = 1, forward shift), dy vx and
+            // dy vz (backward)
+            const float2* T = c == 1 ? k.Fy : k.By;
+            const float inv_n = 1.0f / ((float)n * (float)k.nz);
+            float2* yd = k.Yv[c] + off;
+            auto load_d = [&](int p, int i) -> float2 { return cmul(C[p * n + i], cscale(T[i], inv_n)); };
+            auto store_d = [&](int p, int i, float2 v) {
+                if (p < lv) yd[(long long)p * n + i] = v;
+            };
+            fft_any<N, 8, kCyThreads, kLinePad, true>(k.py, tw, A, B, L, n + n / 16, 1, load_d, store_d);
+        }
+    }
+}
+
+// ------------------------------------------------------------------ k_mx --
+// x-pencils of a (kz, y-chunk) tile in k-space for one velocity component c
+// (blockIdx.z): forward x-FFT of V_c, then the 9 fields that use V_c --
+// 3 derivatives x 3 dispersion operators Ap_j D_d V_c -- each inverse
+// x-transformed on chip.  blockIdx.y + kz0 is the kz plane.
+template <int N>
+__global__ void __launch_bounds__(kThreads) k_mx(KP k, int P_rt, int kz0)
+{
+    extern __shared__ float4 smem4[];
+    float2* sm = reinterpret_cast<float2*>(smem4);
+    const int P = N > 0 ? 16 : P_rt;
+    const int n = N > 0 ? N : k.nx;
+    // the second transform buffer exists only for transforms of more than
+    // two stages (a two-stage transform reads its input through `load` and
+    // writes its output through `store`)
+    const int nbuf = (N > 0 ? ct_nst(N) : k.px.nst) > 2 ? 2 : 1;
+    float2* tw = sm;
+    float2* tFx = tw + n;
+    float2* tBx = tFx + n;
+    float2* V = tBx + n;            // [n][P]
+    float2* A = V + n * P;
+    float2* B = A + (n + n / 16) * P;
+    float2* tFBy = A + nbuf * (n + n / 16) * P;  // [2][P]: Fy, By of the tile's rows
+    float* tkx = reinterpret_cast<float*>(tFBy + 2 * P);
+    float* tky = tkx + n;                         // [P]
+    const int kz = kz0 + blockIdx.y, y0 = blockIdx.x * P, c = blockIdx.z % 3;
+    const int part = blockIdx.z / 3, parts = gridDim.z / 3;  // of the three directions of c
+    const int yv = min(P, k.ny - y0);  // rows of the tile inside the grid
+    load_table(tw, k.tw_x, n);
+    load_table(tFx, k.Fx, n);
+    load_table(tBx, k.Bx, n);
+    for (int i = threadIdx.x; i < n; i += blockDim.x) tkx[i] = k.kx[i];
+    for (int i = threadIdx.x; i < P; i += blockDim.x) {
+        const bool in = i < yv;
+        tky[i] = in ? k.ky[y0 + i] : 0.f;
+        tFBy[i] = in ? k.Fy[y0 + i] : make_float2(0.f, 0.f);
+        tFBy[P + i] = in ? k.By[y0 + i] : make_float2(0.f, 0.f);
+    }
+    __syncthreads();
+
+    {
+        const float2* H = k.Hy[c];
+        auto load = [&](int p, int i) -> float2 { return p < yv ? H[spec(k, kz, i, y0 + p)] : make_float2(0.f, 0.f); };
+        auto store = [&](int p, int i, float2 v) { V[i * P + p] = v; };
+        fft_any<N, 16, kThreads, kPencil, false>(k.px, tw, A, B, P, 1, P, load, store);
+    }
+
+    const float kzv = k.kz[kz];
+    const float kz2 = kzv * kzv;
+    const float2 tFz = k.Fz[kz], tBz = k.Bz[kz];
+    for (int d = 0, nd = 0; d < 9; ++d) {
+        if (c_comp[d] != c || nd++ % parts != part) continue;
+        const int ax = c_axis[d], fw = c_fwd[d];
+        for (int j = 0; j < 3; ++j) {
+            if (is_gz(3 * d + j) || is_gy(3 * d + j)) continue;  // one-axis fields: formed elsewhere
+            float2* G = k.G[3 * d + j];
+            auto load = [&](int p, int i) -> float2 {
+                const float kyv = tky[p];
+                const float kxv = tkx[i];
+                float k2 = kxv * kxv + kyv * kyv + kz2;
+                k2 = fmaxf(k2, 1e-10f);  // the reference sets |k|^2 = 1e-10 at DC (cu:74)
+                // |k|^-1 and |k| from the hardware reciprocal square root
+                // (~2 ulp): far below the FP32 transforms' own rounding
+                const float rk = rsqrtf(k2);
+                const float ap = j == 1 ? 1.0f : (j == 0 ? rk : k2 * rk);
+                float2 T;
+                if (ax == 0) T = fw ? tFx[i] : tBx[i];
+                else if (ax == 1) T = fw ? tFBy[p] : tFBy[P + p];
+                else T = fw ? tFz : tBz;
+                return cmul(V[i * P + p], cscale(T, ap * k.inv_ntp));
+            };
+            auto store = [&](int p, int i, float2 v) {
+                if (p < yv) G[spec(k, kz, i, y0 + p)] = v;
+            };
+            fft_any<N, 16, kThreads, kPencil, true>(k.px, tw, A, B, P, 1, P, load, store);
+        }
+    }
+}
+
+}  // namespace
+
+// Parts k_mx splits each component's directions into: three (the forward
+// transform repeated in each) where one block per component would leave SMs
+// without a block.
+static int mx_parts(const KP& k, int P, int nb) { return cdiv(k.ny, P) * nb * 3 < 2 * 148 ? 3 : 1; }
+
+QVTI_DECLARE_PARTS(bool, fz_launch, const KP& k, int P, int ncomp, cudaStream_t st);
+QVTI_DECLARE_PARTS(bool, cy_launch, const KP& k, int L, bool inv, dim3 grid, size_t sm, long long line0,
+                   long long line_end, cudaStream_t st);
+QVTI_DECLARE_PARTS(bool, mx_launch, const KP& k, int P, int kz0, int nb, cudaStream_t st);
+QVTI_DECLARE_PARTS(bool, sp_configure, SmemLimit& lim);
+
+template <>
+bool fz_launch<QVTI_PART>(const KP& k, int P, int ncomp, cudaStream_t st)
+{
+    return dispatch_len(k.nz, [&](auto NN) {
+        k_fz<decltype(NN)::value><<<dim3(cdiv(k.ny, P), k.nx, ncomp), kThreads, smem_fz(k, P), st>>>(k, P);
+    });
+}
+template <>
+bool cy_launch<QVTI_PART>(const KP& k, int L, bool inv, dim3 grid, size_t sm, long long line0, long long line_end,
+                          cudaStream_t st)
+{
+    return dispatch_len(k.ny, [&](auto NN) {
+        constexpr int N = decltype(NN)::value;
+        if (inv) k_cy<N, true><<<grid, kCyThreads, sm, st>>>(k, L, line0, line_end);
+        else k_cy<N, false><<<grid, kCyThreads, sm, st>>>(k, L, line0, line_end);
+    });
+}
+template <>
+bool mx_launch<QVTI_PART>(const KP& k, int P, int kz0, int nb, cudaStream_t st)
+{
+    return dispatch_len(k.nx, [&](auto NN) {
+        k_mx<decltype(NN)::value><<<dim3(cdiv(k.ny, P), nb, 3 * mx_parts(k, P, nb)), kThreads, smem_mx(k, P), st>>>(k, P, kz0);
+    });
+}
+template <>
+bool sp_configure<QVTI_PART>(SmemLimit& lim)
+{
+    for (int n : kMyLengths)
+        dispatch_len(n, [&](auto NN) {
+            constexpr int N = decltype(NN)::value;
+            lim.set((const void*)k_fz<N>);
+            lim.set((const void*)k_cy<N, false>);
+            lim.set((const void*)k_cy<N, true>);
+            lim.set((const void*)k_mx<N>);
+        });
+    return false;
+}
+
+#if QVTI_PART == 0
+size_t smem_fz(const KP& k, int P) { return sizeof(float2) * (k.nz + 2 * (P / 2) * (k.nz + k.nz / 16)); }
+size_t smem_cy(const KP& k, int L, bool ydv)
+{
+    return sizeof(float2) * (k.ny + 2 * L * (k.ny + k.ny / 16) + (ydv ? (size_t)L * k.ny : 0));
+}
+size_t smem_mx(const KP& k, int P)
+{
+    const int nbuf = k.px.nst > 2 ? 2 : 1;
+    return sizeof(float2) * (3 * k.nx + k.nx * P + nbuf * (k.nx + k.nx / 16) * P + 2 * P) + sizeof(float) * (k.nx + P);
+}
+
+void launch_fz(const KP& k, int P, bool rt, int ncomp, cudaStream_t st)
+{
+    if (rt) k_fz<0><<<dim3(cdiv(k.ny, P), k.nx, ncomp), rt_threads(k.pz, P / 2), smem_fz(k, P), st>>>(k, P);
+    else (void)QVTI_CALL_PARTS(fz_launch, k, P, ncomp, st);
+}
+
+void launch_cy(const KP& k, int L, bool rt, bool inv, int nfield, bool ydv, long long line0, long long line_end,
+               cudaStream_t st)
+{
+    const dim3 grid((unsigned)((line_end - line0 + L - 1) / L), nfield);
+    const size_t sm = smem_cy(k, L, ydv);
+    if (!rt) (void)QVTI_CALL_PARTS(cy_launch, k, L, inv, grid, sm, line0, line_end, st);
+    else if (inv) k_cy<0, true><<<grid, kCyThreads, sm, st>>>(k, L, line0, line_end);
+    else k_cy<0, false><<<grid, kCyThreads, sm, st>>>(k, L, line0, line_end);
+}
+
+void launch_mx(const KP& k, int P, bool rt, int kz0, int nb, cudaStream_t st)
+{
+    if (rt) k_mx<0><<<dim3(cdiv(k.ny, P), nb, 3 * mx_parts(k, P, nb)), rt_threads(k.px, P), smem_mx(k, P), st>>>(k, P, kz0);
+    else (void)QVTI_CALL_PARTS(mx_launch, k, P, kz0, nb, st);
+}
+
+cudaError_t configure_spectral()
+{
+    SmemLimit lim;
+    lim.set((const void*)k_fz<0>);
+    lim.set((const void*)k_cy<0, false>);
+    lim.set((const void*)k_cy<0, true>);
+    lim.set((const void*)k_mx<0>);
+    (void)QVTI_CALL_PARTS(sp_configure, lim);
+    return lim.e;
+}
+#endif  // QVTI_PART == 0
+
+}  // namespace qvti
