@@ -1,11 +1,13 @@
 // Spectral passes of the time step: z transforms of the velocities, y lines,
 // and the k-space x pass with the constant-Q operators.
+#include "fft_pair.cuh"
 #include "step_common.cuh"
 
 namespace qvti {
 
 namespace {
 
+#if QVTI_PART == 0
 // Derivative bookkeeping for the 9 stress-side derivatives d (G index
 // o = 3 d + j): component, axis, forward(1)/backward(0) staggered shift.
 // d: 0 dx vx, 1 dy vy, 2 dz vz (forward shift, kvx_x kvy_y kvz_z),
@@ -14,6 +16,7 @@ namespace {
 __constant__ int c_comp[9] = {0, 1, 2, 0, 2, 0, 1, 1, 2};
 __constant__ int c_axis[9] = {0, 1, 2, 2, 0, 1, 0, 2, 1};
 __constant__ int c_fwd[9] = {1, 1, 1, 0, 0, 0, 0, 0, 0};
+#endif
 // G indices that go through the x and y passes (all but kGz)
 __constant__ int c_gxy[kNumGxy] = {0, 1, 2, 3, 5, 6, 8, 9, 11, 12, 13, 14, 15, 17, 18, 19, 20, 21, 23, 24, 26};
 
@@ -108,22 +111,23 @@ __global__ void __launch_bounds__(kCyThreads) k_cy(KP k, int L_rt, long long lin
     }
 }
 
+#if QVTI_PART == 0
 // ------------------------------------------------------------------ k_mx --
+// The runtime-length kernel (k_mp below is the compiled form).
 // x-pencils of a (kz, y-chunk) tile in k-space for one velocity component c
 // (blockIdx.z): forward x-FFT of V_c, then the 9 fields that use V_c --
 // 3 derivatives x 3 dispersion operators Ap_j D_d V_c -- each inverse
 // x-transformed on chip.  blockIdx.y + kz0 is the kz plane.
-template <int N>
-__global__ void __launch_bounds__(kThreads) k_mx(KP k, int P_rt, int kz0)
+__global__ void __launch_bounds__(kThreads) k_mx(KP k, int P, int kz0)
 {
+    constexpr int N = 0;
     extern __shared__ float4 smem4[];
     float2* sm = reinterpret_cast<float2*>(smem4);
-    const int P = N > 0 ? 16 : P_rt;
-    const int n = N > 0 ? N : k.nx;
+    const int n = k.nx;
     // the second transform buffer exists only for transforms of more than
     // two stages (a two-stage transform reads its input through `load` and
     // writes its output through `store`)
-    const int nbuf = (N > 0 ? ct_nst(N) : k.px.nst) > 2 ? 2 : 1;
+    const int nbuf = k.px.nst > 2 ? 2 : 1;
     float2* tw = sm;
     float2* tFx = tw + n;
     float2* tBx = tFx + n;
@@ -187,6 +191,131 @@ __global__ void __launch_bounds__(kThreads) k_mx(KP k, int P_rt, int kz0)
     }
 }
 
+#endif  // QVTI_PART == 0
+
+// ------------------------------------------------------------------ k_mp --
+// Compiled form of k_mx: the same job on pairs of y rows in packed arithmetic
+// (fft_pair.cuh).  The forward transform's last stage leaves V at exactly the
+// points each inverse's first stage takes, so V stays in registers for all
+// seven fields and only the exchanges of the transforms go through shared
+// memory (k_mx, with V there too, took 0.50 ms at 256^3 against 0.42, 47 against 29
+// us at 96^3, 3.5 against 2.46 ms at 512x512x256).
+constexpr int kMpPairs = 8;  // 16 y: 128-byte rows
+constexpr int mp_threads(int n) { return warps_up(kMpPairs * pair_tasks(n)); }
+constexpr size_t mp_smem(int n) { return 16 * ((size_t)kMpPairs * pair_slots(n) + 2 * (size_t)n) + 4 * (size_t)n; }
+// V and the working butterfly: 8 registers a point (radix 16: 168 registers and
+// three blocks measured 0.418 ms at 256^3, 128 and spills 0.447).
+constexpr int mp_blocks(int n)
+{
+    const int regs = pair_rmax(n) >= 14 ? 168 : pair_rmax(n) >= 10 ? 128 : 96;
+    const int b = 65536 / (regs * mp_threads(n)), m = (int)(220 * 1024 / (mp_smem(n) + 1024));
+    return b < 1 ? 1 : b < m ? b : m;
+}
+
+template <int N>
+__global__ void __launch_bounds__(mp_threads(N), mp_blocks(N)) k_mp(KP k, int kz0)
+{
+    constexpr int PP = kMpPairs, NT = mp_threads(N), RM = pair_rmax(N);
+    using F = PairFFT<N, PP, true, false>;
+    using I = PairFFT<N, PP, true, true>;
+    constexpr int R0 = F::R0, RL = F::RL;
+    extern __shared__ float4 smem4[];
+    f2* buf = reinterpret_cast<f2*>(smem4);
+    float4* tw = smem4 + PP * pair_slots(N);
+    float4* tx = tw + N;                                 // the component's x shift / ntp, doubled like the twiddles
+    float* tk = reinterpret_cast<float*>(tx + N);        // kx^2
+    const int kz = kz0 + blockIdx.y, y0 = blockIdx.x * 2 * PP, c = blockIdx.z % 3, t = threadIdx.x;
+    const int part = blockIdx.z / 3, parts = gridDim.z / 3;  // of the three directions of c
+    const float sc = k.inv_ntp;
+    c2 v[RM], V[RM];
+    int p, j;
+    const bool act0 = F::template task<0>(t, p, j);
+    if (act0) {
+        const int y = y0 + 2 * p;
+        const float4* src = reinterpret_cast<const float4*>(k.Hy[c] + spec(k, kz, j, y));
+        const bool in = y < k.ny;
+#pragma unroll
+        for (int r = 0; r < R0; ++r) {
+            const float4 a = in ? src[(long long)r * (N / R0) * k.ny / 2] : make_float4(0.f, 0.f, 0.f, 0.f);
+            v[r] = c2{pack2(a.x, a.z), pack2(a.y, a.w)};
+        }
+    }
+    {
+        const float2* gf = c == 0 ? k.Fx : k.Bx;
+        for (int i = t; i < N; i += NT) {
+            const float2 w = k.tw_x[i], f = gf[i];
+            const float kx = k.kx[i];
+            tw[i] = make_float4(w.x, w.x, w.y, w.y);
+            tx[i] = make_float4(f.x * sc, f.x * sc, f.y * sc, f.y * sc);
+            tk[i] = kx * kx;
+        }
+    }
+    __syncthreads();
+    F::template first<false>(buf, t, v);
+    F::template finish<false>(TwAll<N>{tw}, buf, t, V);
+
+    int pl, jl, pe, je;
+    const bool actl = F::template task<F::NST - 1>(t, pl, jl);
+    const bool acte = I::template task<I::NST - 1>(t, pe, je);
+    const float kzv = k.kz[kz];
+    // rows of this thread's pair (the same in every stage of a pencil-fast
+    // tile): wavenumbers and y shifts
+    const int y = min(y0 + 2 * pl, k.ny - 2);
+    const float ka = k.ky[y], kb = k.ky[y + 1];
+    const f2 kyz = pack2(ka * ka + kzv * kzv, kb * kb + kzv * kzv);
+    const float2* gy = c == 1 ? k.Fy : k.By;
+    const float2 ya = gy[y], yb = gy[y + 1], zz = (c == 2 ? k.Fz : k.Bz)[kz];
+
+    // seven fields: per axis |k|^-1 and |k|, on the x axis also the identity
+    // operator (the other two have one-axis multipliers and are formed elsewhere)
+#pragma unroll 1
+    for (int f = 0; f < 7; ++f) {
+        const int ax = f < 3 ? 0 : f < 5 ? 1 : 2, jj = f < 3 ? f : 2 * ((f - 3) & 1);
+        if (parts == 3 && ax != part) continue;
+        const int d = c == 0 ? (ax == 0 ? 0 : ax == 1 ? 5 : 3) : c == 1 ? (ax == 0 ? 6 : ax == 1 ? 1 : 7)
+                                                                        : (ax == 0 ? 4 : ax == 1 ? 8 : 2);
+        if (actl) {
+            f2 cx = ax == 1 ? pack2(ya.x * sc, yb.x * sc) : pack2(zz.x * sc, zz.x * sc);
+            f2 cy = ax == 1 ? pack2(ya.y * sc, yb.y * sc) : pack2(zz.y * sc, zz.y * sc);
+#pragma unroll
+            for (int r = 0; r < RL; ++r) {
+                const int i = jl + r * (N / RL);
+                f2 mx = cx, my = cy;
+                if (ax == 0) {
+                    const float4 m = tx[i];
+                    mx = pack2(m.x, m.y);
+                    my = pack2(m.z, m.w);
+                }
+                if (jj != 1) {
+                    const float kx2 = tk[i];
+                    const float2 s2 = unpack2(pack2(kx2, kx2) + kyz);
+                    // the reference sets |k|^2 = 1e-10 at DC (cu:74)
+                    const float a = fmaxf(s2.x, 1e-10f), b = fmaxf(s2.y, 1e-10f);
+                    // |k|^-1 and |k| from the hardware reciprocal square root
+                    // (~2 ulp): far below the FP32 transforms' own rounding
+                    f2 ap = pack2(rsqrtf(a), rsqrtf(b));
+                    if (jj == 2) ap = ap * pack2(a, b);
+                    mx = mx * ap;
+                    my = my * ap;
+                }
+                v[r] = cmul_tw<false>(V[r], mx, my);
+            }
+        }
+        __syncthreads();  // the previous transform's last reads of the exchange
+        I::template first<true>(buf, t, v);
+        I::template finish<true>(TwAll<N>{tw}, buf, t, v);
+        const int ye = y0 + 2 * pe;
+        if (acte && ye < k.ny) {
+            float4* dst = reinterpret_cast<float4*>(k.G[3 * d + jj] + spec(k, kz, je, ye));
+#pragma unroll
+            for (int r = 0; r < R0; ++r) {
+                const float2 x = unpack2(v[r].x), q = unpack2(v[r].y);
+                dst[(long long)r * (N / R0) * k.ny / 2] = make_float4(x.x, q.x, x.y, q.y);
+            }
+        }
+    }
+}
+
 }  // namespace
 
 // Parts k_mx splits each component's directions into: three (the forward
@@ -221,7 +350,8 @@ template <>
 bool mx_launch<QVTI_PART>(const KP& k, int P, int kz0, int nb, cudaStream_t st)
 {
     return dispatch_len(k.nx, [&](auto NN) {
-        k_mx<decltype(NN)::value><<<dim3(cdiv(k.ny, P), nb, 3 * mx_parts(k, P, nb)), kThreads, smem_mx(k, P), st>>>(k, P, kz0);
+        constexpr int N = decltype(NN)::value;
+        k_mp<N><<<dim3(cdiv(k.ny, P), nb, 3 * mx_parts(k, P, nb)), mp_threads(N), mp_smem(N), st>>>(k, kz0);
     });
 }
 template <>
@@ -233,7 +363,7 @@ bool sp_configure<QVTI_PART>(SmemLimit& lim)
             lim.set((const void*)k_fz<N>);
             lim.set((const void*)k_cy<N, false>);
             lim.set((const void*)k_cy<N, true>);
-            lim.set((const void*)k_mx<N>);
+            lim.set((const void*)k_mp<N>);
         });
     return false;
 }
@@ -244,8 +374,9 @@ size_t smem_cy(const KP& k, int L, bool ydv)
 {
     return sizeof(float2) * (k.ny + 2 * L * (k.ny + k.ny / 16) + (ydv ? (size_t)L * k.ny : 0));
 }
-size_t smem_mx(const KP& k, int P)
+size_t smem_mx(const KP& k, int P, bool rt)
 {
+    if (!rt) return mp_smem(k.nx);
     const int nbuf = k.px.nst > 2 ? 2 : 1;
     return sizeof(float2) * (3 * k.nx + k.nx * P + nbuf * (k.nx + k.nx / 16) * P + 2 * P) + sizeof(float) * (k.nx + P);
 }
@@ -268,7 +399,7 @@ void launch_cy(const KP& k, int L, bool rt, bool inv, int nfield, bool ydv, long
 
 void launch_mx(const KP& k, int P, bool rt, int kz0, int nb, cudaStream_t st)
 {
-    if (rt) k_mx<0><<<dim3(cdiv(k.ny, P), nb, 3 * mx_parts(k, P, nb)), rt_threads(k.px, P), smem_mx(k, P), st>>>(k, P, kz0);
+    if (rt) k_mx<<<dim3(cdiv(k.ny, P), nb, 3 * mx_parts(k, P, nb)), rt_threads(k.px, P), smem_mx(k, P, true), st>>>(k, P, kz0);
     else (void)QVTI_CALL_PARTS(mx_launch, k, P, kz0, nb, st);
 }
 
@@ -278,7 +409,7 @@ cudaError_t configure_spectral()
     lim.set((const void*)k_fz<0>);
     lim.set((const void*)k_cy<0, false>);
     lim.set((const void*)k_cy<0, true>);
-    lim.set((const void*)k_mx<0>);
+    lim.set((const void*)k_mx);
     (void)QVTI_CALL_PARTS(sp_configure, lim);
     return lim.e;
 }

@@ -127,7 +127,7 @@ void launch_sigma(const KP& k, int P, bool rt, cudaStream_t st);
 size_t smem_vyx(int n, int P, bool rt);
 size_t smem_fz(const KP& k, int P);
 size_t smem_cy(const KP& k, int L, bool ydv);
-size_t smem_mx(const KP& k, int P);
+size_t smem_mx(const KP& k, int P, bool rt);
 size_t smem_sigma(const KP& k, int P, bool rt);
 // Raise the dynamic shared-memory limit of every instantiation; cudaError_t.
 cudaError_t configure_velocity();

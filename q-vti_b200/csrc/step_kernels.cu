@@ -372,7 +372,7 @@ size_t step_smem_bytes(const KP& k)
     m = std::max(m, smem_vyx(k.nx, T.vx, T.rt[1]));
     m = std::max(m, smem_fz(k, T.fz));
     m = std::max(m, smem_cy(k, T.cy, true));
-    m = std::max(m, smem_mx(k, T.mx));
+    m = std::max(m, smem_mx(k, T.mx, T.rt[4]));
     m = std::max(m, smem_sigma(k, T.sigma, T.rt[5]));
     return m;
 }
