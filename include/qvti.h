@@ -196,13 +196,14 @@ int qvti_q_derivative(qvti_sim* sim, int axis, int fwd, int power, const float* 
  *   d_in, d_out: device arrays of ntx*nty*ntz floats (caller-owned); the
  *   result is written to d_out asynchronously on `stream` (a cudaStream_t,
  *   NULL for the default stream).
- * Nothing is allocated: the scratch half spectrum and the 1D tables live in
- * fixed-size device arrays of the library, held by every GPU that loads it
- * until the process exits.  Limits: each dimension even, 16..1024 and
+ * Nothing is allocated: the scratch half spectrum lives in a fixed-size device
+ * array of the library, held by every GPU that loads it until the process
+ * exits.  Limits: each dimension even, 16..1024 and
  * 2/3/5/7-smooth, and (ntz/2 + 1)*ntx*nty <= 524288 (4 MiB of scratch, e.g.
  * 96^3 or 64x64x128); larger grids return QVTI_ERR_UNSUPPORTED.  The first
- * call on a device looks up the arrays' device addresses (and sets kernel
- * attributes) -- make it before any stream capture.  All calls on a device
+ * call on a device looks up the array's device address (and sets kernel
+ * attributes) -- make it before any stream capture.  One cooperative kernel
+ * launch per call.  All calls on a device
  * share one scratch, which keeps the last call's contents (nothing in it
  * needs clearing): calls that can overlap on the GPU (different streams,
  * no ordering between them) race and must not be issued. */
