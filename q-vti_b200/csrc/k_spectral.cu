@@ -56,22 +56,24 @@ __global__ void __launch_bounds__(kThreads) k_fz(KP k, int P_rt)
     }
 }
 
+#if QVTI_PART == 0
 // ------------------------------------------------------------------ k_cy --
+// The runtime-length kernel (k_cp below is the compiled form).
 // C2C along y, in place, on L contiguous y lines per block (lines (kz, x)
 // starting at line0).  Line-major mapping on a padded tile: each half warp
 // reads or writes 16 consecutive points (128 bytes) of one line, so a warp
 // access touches two lines, and the radix-16 shared-memory stages are
 // conflict-free.  The field is H[0..2] (forward) or G[0..26] (inverse), by
 // blockIdx.y.
-constexpr int kCyThreads = 128;  // L = 8 lines x 256 points = one radix-16 butterfly per thread
+constexpr int kCyThreads = 128;
 
-template <int N, bool INV>
-__global__ void __launch_bounds__(kCyThreads) k_cy(KP k, int L_rt, long long line0, long long line_end)
+template <bool INV>
+__global__ void __launch_bounds__(kCyThreads) k_cy(KP k, int L, long long line0, long long line_end)
 {
+    constexpr int N = 0;
     extern __shared__ float4 smem4[];
     float2* sm = reinterpret_cast<float2*>(smem4);
-    const int L = N > 0 ? 8 : L_rt;
-    const int n = N > 0 ? N : k.ny;
+    const int n = k.ny;
     float2* tw = sm;
     float2* A = tw + n;
     float2* B = A + L * (n + n / 16);
@@ -107,6 +109,88 @@ __global__ void __launch_bounds__(kCyThreads) k_cy(KP k, int L_rt, long long lin
                 if (p < lv) yd[(long long)p * n + i] = v;
             };
             fft_any<N, 8, kCyThreads, kLinePad, true>(k.py, tw, A, B, L, n + n / 16, 1, load_d, store_d);
+        }
+    }
+}
+
+#endif  // QVTI_PART == 0
+
+// ------------------------------------------------------------------ k_cp --
+// Compiled form of k_cy: eight lines as four packed pairs (fft_pair.cuh), the
+// y derivative of the forward pass taken from the registers the transform
+// ends in (reversed radices), as in k_dv.
+constexpr int kCpPairs = 4;
+constexpr int cp_threads(int n) { return warps_up(kCpPairs * pair_tasks(n)); }
+constexpr size_t cp_smem(int n) { return 16 * ((size_t)kCpPairs * pair_slots(n) + tw_rows_size(n)); }
+// (0.56 ms for the inverse pass at 256^3, 5.1 TB/s, where the scalar kernel took
+// 0.54; 1.98 against 3.57 ms at 512x512x256, 48 against 77 us at 96x150x96, and
+// the forward pass 0.10 against 0.135 ms at 256^3.)
+constexpr int cp_blocks(int n)
+{
+    const int warps = cp_threads(n) / 32;
+    int b = 65536 / ((pair_rmax(n) >= 14 ? 128 : pair_rmax(n) >= 10 ? 96 : 80) * cp_threads(n));
+    while (b > 1 && b * warps % 4) --b;
+    return b < 1 ? 1 : b;
+}
+
+template <int N, bool INV>
+__global__ void __launch_bounds__(cp_threads(N), cp_blocks(N)) k_cp(KP k, long long line0, long long line_end)
+{
+    using F = PairFFT<N, kCpPairs, false, false>;
+    constexpr int NT = cp_threads(N), RM = pair_rmax(N), R0 = F::R0, RL = F::RL;
+    extern __shared__ float4 smem4[];
+    f2* buf = reinterpret_cast<f2*>(smem4);
+    float4* tw = smem4 + kCpPairs * pair_slots(N);
+    const int c = blockIdx.y, t = threadIdx.x;
+    const long long first = line0 + (long long)blockIdx.x * 2 * kCpPairs, left = line_end - first;
+    const float2* src = (INV ? k.G[c_gxy[c]] : k.H[c]) + first * N;
+    float2* dst = (INV ? k.G[c_gxy[c]] : k.Hy[c]) + first * N;
+    c2 v[RM];
+    int p, j;
+    if (F::template task<0>(t, p, j)) {
+        const float2* a = src + 2 * p * N + j;
+        const bool in0 = 2 * p < left, in1 = 2 * p + 1 < left;
+#pragma unroll
+        for (int r = 0; r < R0; ++r) {
+            const float2 x = in0 ? a[r * (N / R0)] : make_float2(0.f, 0.f);
+            const float2 y = in1 ? a[r * (N / R0) + N] : make_float2(0.f, 0.f);
+            v[r] = c2{pack2(x.x, y.x), pack2(x.y, y.y)};
+        }
+    }
+    TwRows<N>::template fill<NT>(tw, k.tw_y);
+    F::template first<INV>(buf, t, v);
+    F::template finish<INV>(TwRows<N>{tw}, buf, t, v);
+    auto store = [&](float2* to, int pp, int i, c2 w) {
+        const float2 re = unpack2(w.x), im = unpack2(w.y);
+        if (2 * pp < left) to[2 * pp * N + i] = make_float2(re.x, im.x);
+        if (2 * pp + 1 < left) to[(2 * pp + 1) * N + i] = make_float2(re.y, im.y);
+    };
+    const bool actl = F::template task<F::NST - 1>(t, p, j);
+    if (actl) {
+#pragma unroll
+        for (int r = 0; r < RL; ++r) store(dst, p, j + r * (N / RL), v[r]);
+    }
+    if constexpr (!INV) {
+        // the y derivative with the identity dispersion operator, scaled by
+        // 1/(ny nz) like a field of the x and y passes (1/ntp times the x round
+        // trip's nx): dy vy (c = 1, forward shift), dy vx and dy vz (backward)
+        using I = PairFFT<N, kCpPairs, false, true>;
+        const float2* T = c == 1 ? k.Fy : k.By;
+        const float inv_n = 1.0f / ((float)N * (float)k.nz);
+        if (actl) {
+#pragma unroll
+            for (int r = 0; r < RL; ++r) {
+                const float2 m = cscale(__ldg(T + j + r * (N / RL)), inv_n);
+                v[r] = cmul_tw<false>(v[r], pack2(m.x, m.x), pack2(m.y, m.y));
+            }
+        }
+        __syncthreads();
+        I::template first<true>(buf, t, v);
+        I::template finish<true>(TwGlobal<N>{k.tw_y}, buf, t, v);
+        if (I::template task<I::NST - 1>(t, p, j)) {
+            float2* yd = k.Yv[c] + first * N;
+#pragma unroll
+            for (int r = 0; r < R0; ++r) store(yd, p, j + r * (N / R0), v[r]);
         }
     }
 }
@@ -200,9 +284,11 @@ __global__ void __launch_bounds__(kThreads) k_mx(KP k, int P, int kz0)
 // seven fields and only the exchanges of the transforms go through shared
 // memory (k_mx, with V there too, took 0.50 ms at 256^3 against 0.42, 47 against 29
 // us at 96^3, 3.5 against 2.46 ms at 512x512x256).
-constexpr int kMpPairs = 8;  // 16 y: 128-byte rows
-constexpr int mp_threads(int n) { return warps_up(kMpPairs * pair_tasks(n)); }
-constexpr size_t mp_smem(int n) { return 16 * ((size_t)kMpPairs * pair_slots(n) + 2 * (size_t)n) + 4 * (size_t)n; }
+// 16 y (128-byte rows); 8 where three stages make a block of many small
+// butterflies (512x512x256: 2.23 against 2.46 ms, 384x384x256 1.48 against 1.59).
+constexpr int mp_pairs(int n) { return mp_rows(n) / 2; }
+constexpr int mp_threads(int n) { return warps_up(mp_pairs(n) * pair_tasks(n)); }
+constexpr size_t mp_smem(int n) { return 16 * ((size_t)mp_pairs(n) * pair_slots(n) + 2 * (size_t)n) + 4 * (size_t)n; }
 // V and the working butterfly: 8 registers a point (radix 16: 168 registers and
 // three blocks measured 0.418 ms at 256^3, 128 and spills 0.447).
 constexpr int mp_blocks(int n)
@@ -215,7 +301,7 @@ constexpr int mp_blocks(int n)
 template <int N>
 __global__ void __launch_bounds__(mp_threads(N), mp_blocks(N)) k_mp(KP k, int kz0)
 {
-    constexpr int PP = kMpPairs, NT = mp_threads(N), RM = pair_rmax(N);
+    constexpr int PP = mp_pairs(N), NT = mp_threads(N), RM = pair_rmax(N);
     using F = PairFFT<N, PP, true, false>;
     using I = PairFFT<N, PP, true, true>;
     constexpr int R0 = F::R0, RL = F::RL;
@@ -324,8 +410,8 @@ __global__ void __launch_bounds__(mp_threads(N), mp_blocks(N)) k_mp(KP k, int kz
 static int mx_parts(const KP& k, int P, int nb) { return cdiv(k.ny, P) * nb * 3 < 2 * 148 ? 3 : 1; }
 
 QVTI_DECLARE_PARTS(bool, fz_launch, const KP& k, int P, int ncomp, cudaStream_t st);
-QVTI_DECLARE_PARTS(bool, cy_launch, const KP& k, int L, bool inv, dim3 grid, size_t sm, long long line0,
-                   long long line_end, cudaStream_t st);
+QVTI_DECLARE_PARTS(bool, cy_launch, const KP& k, bool inv, dim3 grid, long long line0, long long line_end,
+                   cudaStream_t st);
 QVTI_DECLARE_PARTS(bool, mx_launch, const KP& k, int P, int kz0, int nb, cudaStream_t st);
 QVTI_DECLARE_PARTS(bool, sp_configure, SmemLimit& lim);
 
@@ -337,13 +423,12 @@ bool fz_launch<QVTI_PART>(const KP& k, int P, int ncomp, cudaStream_t st)
     });
 }
 template <>
-bool cy_launch<QVTI_PART>(const KP& k, int L, bool inv, dim3 grid, size_t sm, long long line0, long long line_end,
-                          cudaStream_t st)
+bool cy_launch<QVTI_PART>(const KP& k, bool inv, dim3 grid, long long line0, long long line_end, cudaStream_t st)
 {
     return dispatch_len(k.ny, [&](auto NN) {
         constexpr int N = decltype(NN)::value;
-        if (inv) k_cy<N, true><<<grid, kCyThreads, sm, st>>>(k, L, line0, line_end);
-        else k_cy<N, false><<<grid, kCyThreads, sm, st>>>(k, L, line0, line_end);
+        if (inv) k_cp<N, true><<<grid, cp_threads(N), cp_smem(N), st>>>(k, line0, line_end);
+        else k_cp<N, false><<<grid, cp_threads(N), cp_smem(N), st>>>(k, line0, line_end);
     });
 }
 template <>
@@ -361,8 +446,8 @@ bool sp_configure<QVTI_PART>(SmemLimit& lim)
         dispatch_len(n, [&](auto NN) {
             constexpr int N = decltype(NN)::value;
             lim.set((const void*)k_fz<N>);
-            lim.set((const void*)k_cy<N, false>);
-            lim.set((const void*)k_cy<N, true>);
+            lim.set((const void*)k_cp<N, false>);
+            lim.set((const void*)k_cp<N, true>);
             lim.set((const void*)k_mp<N>);
         });
     return false;
@@ -370,8 +455,9 @@ bool sp_configure<QVTI_PART>(SmemLimit& lim)
 
 #if QVTI_PART == 0
 size_t smem_fz(const KP& k, int P) { return sizeof(float2) * (k.nz + 2 * (P / 2) * (k.nz + k.nz / 16)); }
-size_t smem_cy(const KP& k, int L, bool ydv)
+size_t smem_cy(const KP& k, int L, bool ydv, bool rt)
 {
+    if (!rt) return cp_smem(k.ny);
     return sizeof(float2) * (k.ny + 2 * L * (k.ny + k.ny / 16) + (ydv ? (size_t)L * k.ny : 0));
 }
 size_t smem_mx(const KP& k, int P, bool rt)
@@ -391,10 +477,10 @@ void launch_cy(const KP& k, int L, bool rt, bool inv, int nfield, bool ydv, long
                cudaStream_t st)
 {
     const dim3 grid((unsigned)((line_end - line0 + L - 1) / L), nfield);
-    const size_t sm = smem_cy(k, L, ydv);
-    if (!rt) (void)QVTI_CALL_PARTS(cy_launch, k, L, inv, grid, sm, line0, line_end, st);
-    else if (inv) k_cy<0, true><<<grid, kCyThreads, sm, st>>>(k, L, line0, line_end);
-    else k_cy<0, false><<<grid, kCyThreads, sm, st>>>(k, L, line0, line_end);
+    const size_t sm = smem_cy(k, L, ydv, true);
+    if (!rt) (void)QVTI_CALL_PARTS(cy_launch, k, inv, grid, line0, line_end, st);
+    else if (inv) k_cy<true><<<grid, kCyThreads, sm, st>>>(k, L, line0, line_end);
+    else k_cy<false><<<grid, kCyThreads, sm, st>>>(k, L, line0, line_end);
 }
 
 void launch_mx(const KP& k, int P, bool rt, int kz0, int nb, cudaStream_t st)
@@ -407,8 +493,8 @@ cudaError_t configure_spectral()
 {
     SmemLimit lim;
     lim.set((const void*)k_fz<0>);
-    lim.set((const void*)k_cy<0, false>);
-    lim.set((const void*)k_cy<0, true>);
+    lim.set((const void*)k_cy<false>);
+    lim.set((const void*)k_cy<true>);
     lim.set((const void*)k_mx);
     (void)QVTI_CALL_PARTS(sp_configure, lim);
     return lim.e;

@@ -115,6 +115,9 @@ inline int rt_threads(const FftPlan& p, int pencils)
 
 inline int cdiv(int a, int b) { return (a + b - 1) / b; }
 
+// y rows of a compiled k_mx block.
+__host__ __device__ constexpr int mp_rows(int n) { return radix_seq(n).nst > 2 ? 8 : 16; }
+
 // One kernel of the step: tile `P`, rt = the runtime-length kernel.
 void launch_vy(const KP& k, int P, bool rt, cudaStream_t st);
 void launch_vx(const KP& k, int P, bool rt, cudaStream_t st);
@@ -126,7 +129,7 @@ void launch_sigma(const KP& k, int P, bool rt, cudaStream_t st);
 // Their dynamic shared memory (bytes).
 size_t smem_vyx(int n, int P, bool rt);
 size_t smem_fz(const KP& k, int P);
-size_t smem_cy(const KP& k, int L, bool ydv);
+size_t smem_cy(const KP& k, int L, bool ydv, bool rt);
 size_t smem_mx(const KP& k, int P, bool rt);
 size_t smem_sigma(const KP& k, int P, bool rt);
 // Raise the dynamic shared-memory limit of every instantiation; cudaError_t.

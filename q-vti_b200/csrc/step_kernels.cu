@@ -299,6 +299,7 @@ StepTiles step_tiles(const KP& k)
     t.fz = tile(2, k.nz, k.ny, 16);
     t.cy = tile(3, k.ny, k.nx, 8);
     t.mx = tile(4, k.nx, k.ny, 16);
+    if (!t.rt[4]) t.mx = mp_rows(k.nx);
     t.sigma = tile(5, k.nz, k.ny, kSigmaRows);
     return t;
 }
@@ -371,7 +372,7 @@ size_t step_smem_bytes(const KP& k)
     size_t m = smem_vyx(k.ny, T.vy, T.rt[0]);
     m = std::max(m, smem_vyx(k.nx, T.vx, T.rt[1]));
     m = std::max(m, smem_fz(k, T.fz));
-    m = std::max(m, smem_cy(k, T.cy, true));
+    m = std::max(m, smem_cy(k, T.cy, true, T.rt[3]));
     m = std::max(m, smem_mx(k, T.mx, T.rt[4]));
     m = std::max(m, smem_sigma(k, T.sigma, T.rt[5]));
     return m;
