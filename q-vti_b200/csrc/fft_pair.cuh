@@ -63,6 +63,16 @@ __host__ __device__ constexpr int pair_slots(int n)
     return n + (pair_pad(n, false) > pair_pad(n, true) ? pair_pad(n, false) : pair_pad(n, true));
 }
 
+// Pairs on neighbouring lanes (Q = 2): eight butterflies of each make up a
+// 16-lane access, so the pairs' slots start half of the banks apart.
+__host__ __device__ constexpr int pair_slots_q(int n, int q)
+{
+    int s = pair_slots(n);
+    if (q == 2)
+        while (s % 16 != 8) ++s;
+    return s;
+}
+
 // Twiddles e^{-2 pi i e / N}, e = jm r N / (NS R) in stage S, as (c, c, s, s).
 // TwAll: a shared-memory table of all N (pencil-fast tiles: the lanes of one
 // butterfly read one entry).  TwRows: per stage rows r = 1 .. R-1 of NS
@@ -123,15 +133,17 @@ struct TwGlobal {
     }
 };
 
-// N points, PP pencil pairs per block.
-template <int N, int PP, bool PF, bool REV>
+// N points, PP pencil pairs per block.  Q > 1 (line-major): Q neighbouring
+// pairs on neighbouring lanes, for pencils that share memory lines.
+template <int N, int PP, bool PF, bool REV, int Q = 1>
 struct PairFFT {
     static constexpr int NST = radix_seq(N).nst;
     static constexpr int R0 = pair_rad(N, 0, REV), RL = pair_rad(N, NST - 1, REV);
     template <int S>
     static constexpr int rad() { return pair_rad(N, S, REV); }
 
-    static constexpr int PLANE = PP * pair_slots(N);  // words of one plane
+    static constexpr int SL = pair_slots_q(N, Q);
+    static constexpr int PLANE = PP * SL;  // words of one plane
     static __device__ __forceinline__ void st(f2* b, c2 v)
     {
         b[0] = v.x;
@@ -145,7 +157,8 @@ struct PairFFT {
         constexpr unsigned NR = N / pair_rad(N, S, REV);
         const unsigned u = t;
         if constexpr (PF) { p = u % PP; j = u / PP; }
-        else { p = u / NR; j = u % NR; }
+        else if constexpr (Q == 1) { p = u / NR; j = u % NR; }
+        else { p = u / (Q * NR) * Q + u % Q; j = u / Q % NR; }
         return u < PP * NR;
     }
     // Slots: one pad per R0 indices where R0 is even.  Every stage's accesses
@@ -157,7 +170,6 @@ struct PairFFT {
     static __device__ __forceinline__ int slot(int p, int i)
     {
         const int q = PAD ? i + (int)((unsigned)i / R0) : i;
-        constexpr int SL = pair_slots(N);
         return PF ? q * PP + p : p * SL + q;
     }
     // Slot of point r of stage S's butterfly j (S >= 1; its inputs, and the

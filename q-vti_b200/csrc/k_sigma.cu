@@ -31,15 +31,18 @@ __device__ __forceinline__ void prefetch_l2(const void* p, unsigned bytes)
 // measured 0.72 against 0.57 ms for the normal stresses), those
 // above are the mirror of what the butterfly n/R - j loaded and come by
 // shuffle where the butterflies of a pencil are 8 or 16 neighbouring lanes (a
-// second load otherwise: 2.65 against 2.2 ms).
-constexpr int st_threads(int n, int nf) { return warps_up(nf * pair_tasks(n)); }
-constexpr size_t st_smem(int n, int nf) { return 16 * ((size_t)nf * pair_slots(n) + tw_rows_size(n)); }
-// Blocks per SM the registers are sized for.
-template <int N, int NF>
-constexpr int st_blocks()
+// second load otherwise: 2.65 against 2.2 ms).  With eight rows (Q = 2) the two
+// row quads of a butterfly are neighbouring lanes and read 64 bytes of a line
+// between them: a warp's load touches 16 lines instead of 32 (shear 0.68
+// against 0.78 ms at 256^3, the whole update 1.40 against 1.52).
+constexpr int st_threads(int n, int nf, int q) { return warps_up(nf * q * pair_tasks(n)); }
+constexpr size_t st_smem(int n, int nf, int q) { return 16 * ((size_t)nf * q * pair_slots_q(n, q) + tw_rows_size(n)); }
+// Blocks per SM the registers are sized for (256 points, normal stresses: two
+// blocks of nine warps at 96 registers 0.536 ms, one at 158 0.577).
+constexpr int st_blocks(int n, int nf, int q)
 {
-    const int warps = st_threads(N, NF) / 32, m = (int)(200 * 1024 / (st_smem(N, NF) + 2048));
-    int b = (NF == 9 ? 16 : 20) / warps;
+    const int warps = st_threads(n, nf, q) / 32, m = (int)(220 * 1024 / (st_smem(n, nf, q) + 2048));
+    int b = (nf == 9 ? (q == 1 ? 16 : 18) : 20) / warps;
     if (b < 1) b = 1;
     return b < m ? b : m < 1 ? 1 : m;
 }
@@ -329,20 +332,20 @@ __device__ __forceinline__ void stress_pair(const KP& k, int n, int grp, int x, 
     }
 }
 
-template <int N, int NF>
-__global__ void __launch_bounds__(st_threads(N, NF), st_blocks<N, NF>()) k_st(KP k)
+template <int N, int NF, int Q>
+__global__ void __launch_bounds__(st_threads(N, NF, Q), st_blocks(N, NF, Q)) k_st(KP k)
 {
-    using F = PairFFT<N, NF, false, false>;
-    constexpr int NT = st_threads(N, NF), R0 = F::R0, RL = F::RL, NR0 = N / R0, SL = pair_slots(N);
-    constexpr bool SHFL = R0 % 2 == 0 && (NR0 == 8 || NR0 == 16);
+    using F = PairFFT<N, NF * Q, false, false, Q>;
+    constexpr int NT = st_threads(N, NF, Q), R0 = F::R0, RL = F::RL, NR0 = N / R0, ROWS = 4 * Q;
+    constexpr bool SHFL = R0 % 2 == 0 && (NR0 * Q == 8 || NR0 * Q == 16 || NR0 * Q == 32);
     constexpr int RM = pair_rmax(N);
     extern __shared__ float4 smem4[];
     f2* buf = reinterpret_cast<f2*>(smem4);
-    float4* tw = smem4 + NF * SL;
+    float4* tw = smem4 + F::PLANE;
     const int t = threadIdx.x, nx = k.nx, ny = k.ny, x = blockIdx.y;
     // the three shear blocks of a tile are neighbours: they share MU in L2
-    const int y0 = 4 * (NF == 9 ? blockIdx.x : blockIdx.x / 3);
-    const int yv = min(4, ny - y0);  // rows of the tile inside the grid: 4 or 2
+    const int y0 = ROWS * (NF == 9 ? blockIdx.x : blockIdx.x / 3);
+    const int yv = min(ROWS, ny - y0);  // rows of the tile inside the grid (even)  // rows of the tile inside the grid: 4 or 2
     constexpr float inv_nz = 1.0f / N;
     const int grp = NF == 9 ? 0 : blockIdx.x % 3 + 1;
     if (x == nx - 1) {  // the last plane of an axis is never updated
@@ -351,27 +354,29 @@ __global__ void __launch_bounds__(st_threads(N, NF), st_blocks<N, NF>()) k_st(KP
     }
 
     if (t == 0) prefetch_group(k, N, grp, x, y0, yv);
-    int f0, j0;
-    const bool act0 = F::template task<0>(t, f0, j0);
-    if (!act0) { f0 = NF - 1; j0 = t % NR0; } 
+    int p0, j0;
+    const bool act0 = F::template task<0>(t, p0, j0);
+    if (!act0) { p0 = NF * Q - Q + t % Q; j0 = t / Q % NR0; }
+    const int f0 = p0 / Q, q0 = 4 * (p0 % Q);  // field and first row of the pair 
 
     c2 v[RM];
     // 1. C2R along z of the group's fields (whole warps: lanes past the
     //    last butterfly follow along for the shuffles)
-    if ((t & ~31) < NF * NR0) {
+    if ((t & ~31) < NF * Q * NR0) {
         const int o = (NF == 9 ? 0 : 3 + 6 * grp) + f0;
         const bool gz = is_gz(o);
         const float2* src = gz ? k.H[o == 7 ? 2 : o == 10 ? 0 : 1]
                                : is_gy(o) ? k.Yv[o == 4 ? 1 : o == 16 ? 0 : 2] : k.G[o];
         const float2* M = o == 7 ? k.Fz : k.Bz;
-        src += (long long)x * ny + y0;
+        const bool r01 = q0 < yv, r23 = q0 + 2 < yv;
+        src += (long long)x * ny + y0 + (r01 ? q0 : 0);
         const int ks = nx * ny;
         // the four rows at kz, the kz-only fields' multiplier applied
         // (imaginary parts dropped at kz = 0 and n/2 like a C2R)
         auto rows = [&](int kk, float2 a[4]) {
             const float2* at = src + (long long)kk * ks;
             const float4 u = *reinterpret_cast<const float4*>(at);
-            const float4 w = yv == 4 ? *reinterpret_cast<const float4*>(at + 2) : make_float4(0.f, 0.f, 0.f, 0.f);
+            const float4 w = r23 ? *reinterpret_cast<const float4*>(at + 2) : make_float4(0.f, 0.f, 0.f, 0.f);
             a[0] = make_float2(u.x, u.y); a[1] = make_float2(u.z, u.w);
             a[2] = make_float2(w.x, w.y); a[3] = make_float2(w.z, w.w);
             if (gz) {
@@ -399,10 +404,10 @@ __global__ void __launch_bounds__(st_threads(N, NF), st_blocks<N, NF>()) k_st(KP
                 v[r] = direct(a);
                 m[r] = mirror(a);
             }
-            const int from = NR0 - j0;  // the butterfly that holds the mirror points (lane 0: itself)
+            const int from = (NR0 - j0) * Q + p0 % Q;  // the butterfly that holds the mirror points (lane 0: itself)
             auto swap1 = [&](f2 own, f2 send) {
                 const float2 s = unpack2(send), w = unpack2(own);
-                const float p = __shfl_sync(0xffffffffu, s.x, from, NR0), q = __shfl_sync(0xffffffffu, s.y, from, NR0);
+                const float p = __shfl_sync(0xffffffffu, s.x, from, NR0 * Q), q = __shfl_sync(0xffffffffu, s.y, from, NR0 * Q);
                 return j0 ? pack2(p, q) : pack2(w.x, w.y);
             };
             c2 ny2 = m[0];
@@ -441,11 +446,11 @@ __global__ void __launch_bounds__(st_threads(N, NF), st_blocks<N, NF>()) k_st(KP
     __syncthreads();
 
     // 2. stress update of the group: a thread takes rows 2h, 2h + 1 at z
-    for (int w = t; w < 2 * N; w += NT) {
+    for (int w = t; w < ROWS / 2 * N; w += NT) {
         const int h = (unsigned)w / N, z = w - h * N, y = y0 + 2 * h;
         if (2 * h >= yv || z == N - 1) continue;
-        const f2* S = buf + h * F::PLANE + F::slot(0, z);
-        stress_pair(k, N, grp, x, y, z, [&](int f) { return S[f * SL]; });
+        const f2* S = buf + (h & 1) * F::PLANE + F::slot(h / 2, z);
+        stress_pair(k, N, grp, x, y, z, [&](int f) { return S[f * Q * F::SL]; });
     }
     if constexpr (NF == 9) {
         __syncthreads();
@@ -636,17 +641,29 @@ __global__ void __launch_bounds__(kThreads) k_dzr(KP k, int P)
 
 }  // namespace
 
-QVTI_DECLARE_PARTS(bool, st_launch, const KP& k, cudaStream_t st);
+QVTI_DECLARE_PARTS(bool, st_launch, const KP& k, int P, cudaStream_t st);
 QVTI_DECLARE_PARTS(bool, st_configure, SmemLimit& lim);
 
 template <>
-bool st_launch<QVTI_PART>(const KP& k, cudaStream_t st)
+bool st_launch<QVTI_PART>(const KP& k, int P, cudaStream_t st)
 {
     return dispatch_len(k.nz, [&](auto NN) {
         constexpr int N = decltype(NN)::value;
-        const int tiles = cdiv(k.ny, kSigmaRows);
-        k_st<N, 9><<<dim3(tiles, k.nx), st_threads(N, 9), st_smem(N, 9), st>>>(k);
-        k_st<N, 6><<<dim3(3 * tiles, k.nx), st_threads(N, 6), st_smem(N, 6), st>>>(k);
+        const int tiles = cdiv(k.ny, P);
+        auto go = [&](auto QQ) {
+            constexpr int q = decltype(QQ)::value;
+            k_st<N, 9, q><<<dim3(tiles, k.nx), st_threads(N, 9, q), st_smem(N, 9, q), st>>>(k);
+            k_st<N, 6, q><<<dim3(3 * tiles, k.nx), st_threads(N, 6, q), st_smem(N, 6, q), st>>>(k);
+        };
+        if constexpr (st_eight_rows(N)) {
+            if (P == 8) {
+                go(IntC<2>{});
+            } else {
+                go(IntC<1>{});
+            }
+        } else {
+            go(IntC<1>{});
+        }
         k_dz<N><<<dim3(cdiv(k.ny, 4 * kDzPairs), k.nx, 3), dz_threads(N), dz_smem(N), st>>>(k);
     });
 }
@@ -656,8 +673,12 @@ bool st_configure<QVTI_PART>(SmemLimit& lim)
     for (int n : kMyLengths)
         dispatch_len(n, [&](auto NN) {
             constexpr int N = decltype(NN)::value;
-            lim.set((const void*)k_st<N, 9>);
-            lim.set((const void*)k_st<N, 6>);
+            lim.set((const void*)k_st<N, 9, 1>);
+            lim.set((const void*)k_st<N, 6, 1>);
+            if constexpr (st_eight_rows(N)) {
+                lim.set((const void*)k_st<N, 9, 2>);
+                lim.set((const void*)k_st<N, 6, 2>);
+            }
             lim.set((const void*)k_dz<N>);
         });
     return false;
@@ -668,7 +689,7 @@ bool st_configure<QVTI_PART>(SmemLimit& lim)
 // S[9][P][nz+1]; k_dzr's tw | A | B is smaller.
 size_t smem_sigma(const KP& k, int P, bool rt)
 {
-    if (!rt) return std::max(st_smem(k.nz, 9), dz_smem(k.nz));
+    if (!rt) return std::max(st_smem(k.nz, 9, P / 4), dz_smem(k.nz));
     const size_t bufA = (size_t)9 * (P / 2) * (k.nz + k.nz / 16);
     const int nb = k.pz.nst > 2 ? 2 : 1;
     return sizeof(float2) * (k.nz + nb * bufA) + sizeof(float) * (size_t)9 * P * (k.nz + 1);
@@ -677,7 +698,7 @@ size_t smem_sigma(const KP& k, int P, bool rt)
 void launch_sigma(const KP& k, int P, bool rt, cudaStream_t st)
 {
     if (!rt) {
-        (void)QVTI_CALL_PARTS(st_launch, k, st);
+        (void)QVTI_CALL_PARTS(st_launch, k, P, st);
         return;
     }
     const int tiles = cdiv(k.ny, P);

@@ -118,6 +118,11 @@ inline int cdiv(int a, int b) { return (a + b - 1) / b; }
 // y rows of a compiled k_mx block.
 __host__ __device__ constexpr int mp_rows(int n) { return radix_seq(n).nst > 2 ? 8 : 16; }
 
+// Lengths whose compiled stress kernels also come with eight rows: those of two
+// stages (three have up to 64 butterflies a pencil, and eighteen pencils would
+// pass the threads of a block).
+__host__ __device__ constexpr bool st_eight_rows(int n) { return radix_seq(n).nst == 2; }
+
 // One kernel of the step: tile `P`, rt = the runtime-length kernel.
 void launch_vy(const KP& k, int P, bool rt, cudaStream_t st);
 void launch_vx(const KP& k, int P, bool rt, cudaStream_t st);

@@ -279,6 +279,12 @@ bool ct_length(int n)
 // for k_vy, 0.34 against 0.22 for k_vx at 256^3) unless that leaves fewer than
 // two blocks per SM.
 int dv_tile(int nz, int lines) { return nz % 4 || 3ll * cdiv(nz, 32) * lines >= 2 * 148 ? 32 : 16; }
+// The compiled stress kernels take eight rows (half-line accesses, see k_st)
+// unless that leaves fewer than four blocks per SM.
+int st_rows(const KP& k)
+{
+    return st_eight_rows(k.nz) && (long long)cdiv(k.ny, 8) * k.nx >= 4 * 148 ? 8 : kSigmaRows;
+}
 struct StepTiles {
     int vy, vx, fz, cy, mx, sigma;
     bool rt[kNumTiled];  // runtime path, in the order above
@@ -301,6 +307,7 @@ StepTiles step_tiles(const KP& k)
     t.mx = tile(4, k.nx, k.ny, 16);
     if (!t.rt[4]) t.mx = mp_rows(k.nx);
     t.sigma = tile(5, k.nz, k.ny, kSigmaRows);
+    if (!t.rt[5]) t.sigma = st_rows(k);
     return t;
 }
 
