@@ -378,16 +378,6 @@ __global__ void __launch_bounds__(dv_threads(N, PP), dv_blocks(N, PP)) k_dv(KP k
     f2* buf = reinterpret_cast<f2*>(smem4);
     float4* tw = smem4 + PP * pair_slots(N);
     float4* tf = tw + N;  // forward shift over n, doubled like the twiddles; the backward one is (-F.x, F.y)
-    {
-        const float2* gtw = AX ? k.tw_y : k.tw_x;
-        const float2* gf = AX ? k.Fy : k.Fx;
-        constexpr float inv_n = 1.0f / N;
-        for (int i = threadIdx.x; i < N; i += NT) {
-            const float2 w = gtw[i], f = gf[i];
-            tw[i] = make_float4(w.x, w.x, w.y, w.y);
-            tf[i] = make_float4(f.x * inv_n, f.x * inv_n, f.y * inv_n, f.y * inv_n);
-        }
-    }
     if (AX == 1 && blockIdx.x + blockIdx.y + blockIdx.z == 0 && threadIdx.x == 0) *k.d_it += 1;  // step counter
     const int t = threadIdx.x, nz = k.nz, pml = k.pml;
     const int line = blockIdx.y;  // x (AX = 1) or y
@@ -436,6 +426,16 @@ __global__ void __launch_bounds__(dv_threads(N, PP), dv_blocks(N, PP)) k_dv(KP k
                     prefetch_line(ri + ip);
                 }
                 if (lin && in_slab(i, N, pml)) prefetch_line(ph + (AX ? slab_y(k, line, i, ze) : slab_x(k, i, line, ze)));
+            }
+        }
+        {  // tables, behind the loads in flight (read after the exchange's barrier)
+            const float2* gtw = AX ? k.tw_y : k.tw_x;
+            const float2* gf = AX ? k.Fy : k.Fx;
+            constexpr float inv_n = 1.0f / N;
+            for (int i = threadIdx.x; i < N; i += NT) {
+                const float2 w = gtw[i], f = gf[i];
+                tw[i] = make_float4(w.x, w.x, w.y, w.y);
+                tf[i] = make_float4(f.x * inv_n, f.x * inv_n, f.y * inv_n, f.y * inv_n);
             }
         }
         F::template first<false>(buf, t, v);

@@ -47,8 +47,11 @@ __device__ __forceinline__ float2* out_any(const FftPlan& pl, float2* A, float2*
 
 // Transform lengths with a compile-time path: the 5-smooth lengths the
 // batching and serving workloads draw between 96 and 384, 512, and the other
-// even 7-smooth lengths from 36 up to the serving range; a kernel takes it
-// when its transform length is listed, otherwise the runtime path.
+// even 7-smooth lengths from 24 up to the serving range; a kernel takes it
+// when its transform length is listed, otherwise the runtime path.  The x
+// kernels (k_vx, k_mx) start at 36: the tile tests run their runtime form at
+// 32.
+constexpr int kMinCtX = 36;
 //
 // The lengths are split into QVTI_PARTS lists: each unit of compiled kernels is
 // built once per list (QVTI_PART), in parallel.
@@ -56,7 +59,7 @@ __device__ __forceinline__ float2* out_any(const FftPlan& pl, float2* A, float2*
 #define QVTI_LENGTHS0(X) X(36) X(48) X(56) X(72) X(90) X(100) X(120) X(140) X(160) X(180) X(200) X(224) X(252) X(288) X(324)
 #define QVTI_LENGTHS1(X) X(40) X(50) X(60) X(80) X(96) X(108) X(126) X(144) X(162) X(192) X(210) X(240) X(256) X(300) X(360)
 #define QVTI_LENGTHS2(X) X(42) X(54) X(64) X(84) X(98) X(112) X(128) X(150) X(168) X(196) X(216) X(250) X(270) X(320) X(384)
-#define QVTI_LENGTHS3(X) X(70) X(512)
+#define QVTI_LENGTHS3(X) X(24) X(28) X(30) X(32) X(70) X(512)
 #define QVTI_LENGTHS(X) QVTI_LENGTHS0(X) QVTI_LENGTHS1(X) QVTI_LENGTHS2(X) QVTI_LENGTHS3(X)
 #define QVTI_ITEM(N) N,
 inline constexpr int kCtLengths[] = {QVTI_LENGTHS(QVTI_ITEM)};

@@ -297,7 +297,7 @@ StepTiles step_tiles(const KP& k)
             t.rt[i] = true;
             return k.tile_rt[i];
         }
-        t.rt[i] = !ct_length(len);
+        t.rt[i] = !ct_length(len) || ((i == 1 || i == 4) && len < kMinCtX);
         return t.rt[i] ? tile_of(tiled, std::min(want, 16)) : want;
     };
     t.vy = tile(0, k.ny, k.nz, dv_tile(k.nz, k.nx));
