@@ -649,22 +649,24 @@ bool st_launch<QVTI_PART>(const KP& k, int P, cudaStream_t st)
 {
     return dispatch_len(k.nz, [&](auto NN) {
         constexpr int N = decltype(NN)::value;
-        const int tiles = cdiv(k.ny, P);
-        auto go = [&](auto QQ) {
-            constexpr int q = decltype(QQ)::value;
-            k_st<N, 9, q><<<dim3(tiles, k.nx), st_threads(N, 9, q), st_smem(N, 9, q), st>>>(k);
-            k_st<N, 6, q><<<dim3(3 * tiles, k.nx), st_threads(N, 6, q), st_smem(N, 6, q), st>>>(k);
-        };
-        if constexpr (st_eight_rows(N)) {
-            if (P == 8) {
-                go(IntC<2>{});
+        if constexpr (N >= kMinLong) {
+            const int tiles = cdiv(k.ny, P);
+            auto go = [&](auto QQ) {
+                constexpr int q = decltype(QQ)::value;
+                k_st<N, 9, q><<<dim3(tiles, k.nx), st_threads(N, 9, q), st_smem(N, 9, q), st>>>(k);
+                k_st<N, 6, q><<<dim3(3 * tiles, k.nx), st_threads(N, 6, q), st_smem(N, 6, q), st>>>(k);
+            };
+            if constexpr (st_eight_rows(N)) {
+                if (P == 8) {
+                    go(IntC<2>{});
+                } else {
+                    go(IntC<1>{});
+                }
             } else {
                 go(IntC<1>{});
             }
-        } else {
-            go(IntC<1>{});
+            k_dz<N><<<dim3(cdiv(k.ny, 4 * kDzPairs), k.nx, 3), dz_threads(N), dz_smem(N), st>>>(k);
         }
-        k_dz<N><<<dim3(cdiv(k.ny, 4 * kDzPairs), k.nx, 3), dz_threads(N), dz_smem(N), st>>>(k);
     });
 }
 template <>
@@ -673,13 +675,15 @@ bool st_configure<QVTI_PART>(SmemLimit& lim)
     for (int n : kMyLengths)
         dispatch_len(n, [&](auto NN) {
             constexpr int N = decltype(NN)::value;
-            lim.set((const void*)k_st<N, 9, 1>);
-            lim.set((const void*)k_st<N, 6, 1>);
-            if constexpr (st_eight_rows(N)) {
-                lim.set((const void*)k_st<N, 9, 2>);
-                lim.set((const void*)k_st<N, 6, 2>);
+            if constexpr (N >= kMinLong) {
+                lim.set((const void*)k_st<N, 9, 1>);
+                lim.set((const void*)k_st<N, 6, 1>);
+                if constexpr (st_eight_rows(N)) {
+                    lim.set((const void*)k_st<N, 9, 2>);
+                    lim.set((const void*)k_st<N, 6, 2>);
+                }
+                lim.set((const void*)k_dz<N>);
             }
-            lim.set((const void*)k_dz<N>);
         });
     return false;
 }

@@ -436,7 +436,8 @@ bool mx_launch<QVTI_PART>(const KP& k, int P, int kz0, int nb, cudaStream_t st)
 {
     return dispatch_len(k.nx, [&](auto NN) {
         constexpr int N = decltype(NN)::value;
-        k_mp<N><<<dim3(cdiv(k.ny, P), nb, 3 * mx_parts(k, P, nb)), mp_threads(N), mp_smem(N), st>>>(k, kz0);
+        if constexpr (N >= kMinLong)
+            k_mp<N><<<dim3(cdiv(k.ny, P), nb, 3 * mx_parts(k, P, nb)), mp_threads(N), mp_smem(N), st>>>(k, kz0);
     });
 }
 template <>
@@ -448,7 +449,7 @@ bool sp_configure<QVTI_PART>(SmemLimit& lim)
             lim.set((const void*)k_fz<N>);
             lim.set((const void*)k_cp<N, false>);
             lim.set((const void*)k_cp<N, true>);
-            lim.set((const void*)k_mp<N>);
+            if constexpr (N >= kMinLong) lim.set((const void*)k_mp<N>);
         });
     return false;
 }

@@ -512,8 +512,11 @@ bool dv_launch<QVTI_PART>(const KP& k, int ax, int P, cudaStream_t st)
             else if (P == 16) k_dv<N, 4, ax_, true><<<grid, dv_threads(N, 4), sm, st>>>(k);
             else k_dv<N, 8, ax_, true><<<grid, dv_threads(N, 8), sm, st>>>(k);
         };
-        if (ax) go(IntC<1>{});
-        else go(IntC<0>{});
+        if (ax) {
+            go(IntC<1>{});
+        } else {
+            if constexpr (N >= kMinLong) go(IntC<0>{});
+        }
     });
 }
 template <>
@@ -522,12 +525,14 @@ bool dv_configure<QVTI_PART>(SmemLimit& lim)
     for (int n : kMyLengths)
         dispatch_len(n, [&](auto NN) {
             constexpr int N = decltype(NN)::value;
-            lim.set((const void*)k_dv<N, 8, 0, true>);
             lim.set((const void*)k_dv<N, 8, 1, true>);
-            lim.set((const void*)k_dv<N, 4, 0, true>);
             lim.set((const void*)k_dv<N, 4, 1, true>);
-            lim.set((const void*)k_dv<N, 8, 0, false>);
             lim.set((const void*)k_dv<N, 8, 1, false>);
+            if constexpr (N >= kMinLong) {
+                lim.set((const void*)k_dv<N, 8, 0, true>);
+                lim.set((const void*)k_dv<N, 4, 0, true>);
+                lim.set((const void*)k_dv<N, 8, 0, false>);
+            }
         });
     return false;
 }

@@ -48,10 +48,12 @@ __device__ __forceinline__ float2* out_any(const FftPlan& pl, float2* A, float2*
 // Transform lengths with a compile-time path: the 5-smooth lengths the
 // batching and serving workloads draw between 96 and 384, 512, and the other
 // even 7-smooth lengths from 24 up to the serving range; a kernel takes it
-// when its transform length is listed, otherwise the runtime path.  The x
-// kernels (k_vx, k_mx) start at 36: the tile tests run their runtime form at
-// 32.
-constexpr int kMinCtX = 36;
+// when its transform length is listed, otherwise the runtime path.  The
+// shortest lengths, below 36, come for k_vy, k_fz and k_cy only: the tile tests
+// run the x kernels' runtime form at 32, and the stress update of so short a z
+// axis is faster in its runtime form with 16 rows per block (32^3: 26 us) than
+// as the compiled kernels' three launches (28).
+constexpr int kMinLong = 36;
 //
 // The lengths are split into QVTI_PARTS lists: each unit of compiled kernels is
 // built once per list (QVTI_PART), in parallel.

@@ -297,7 +297,7 @@ StepTiles step_tiles(const KP& k)
             t.rt[i] = true;
             return k.tile_rt[i];
         }
-        t.rt[i] = !ct_length(len) || ((i == 1 || i == 4) && len < kMinCtX);
+        t.rt[i] = !ct_length(len) || ((i == 1 || i == 4 || i == 5) && len < kMinLong);
         return t.rt[i] ? tile_of(tiled, std::min(want, 16)) : want;
     };
     t.vy = tile(0, k.ny, k.nz, dv_tile(k.nz, k.nx));
@@ -306,7 +306,7 @@ StepTiles step_tiles(const KP& k)
     t.cy = tile(3, k.ny, k.nx, 8);
     t.mx = tile(4, k.nx, k.ny, 16);
     if (!t.rt[4]) t.mx = mp_rows(k.nx);
-    t.sigma = tile(5, k.nz, k.ny, kSigmaRows);
+    t.sigma = tile(5, k.nz, k.ny, k.nz < kMinLong ? 16 : kSigmaRows);
     if (!t.rt[5]) t.sigma = st_rows(k);
     return t;
 }
