@@ -353,7 +353,6 @@ __global__ void __launch_bounds__(st_threads(N, NF, Q), st_blocks(N, NF, Q)) k_s
         return;
     }
 
-    if (t == 0) prefetch_group(k, N, grp, x, y0, yv);
     int p0, j0;
     const bool act0 = F::template task<0>(t, p0, j0);
     if (!act0) { p0 = NF * Q - Q + t % Q; j0 = t / Q % NR0; }
@@ -431,7 +430,10 @@ __global__ void __launch_bounds__(st_threads(N, NF, Q), st_blocks(N, NF, Q)) k_s
             }
         }
     }
-    TwRows<N>::template fill<NT>(tw, k.tw_z);  // behind the loads in flight
+    // behind the loads in flight (ahead of them its dozens of requests held up
+    // the first warp: 1.40 against 1.38 ms at 256^3, 130 against 119 us at 96^3)
+    if (t == 0) prefetch_group(k, N, grp, x, y0, yv);
+    TwRows<N>::template fill<NT>(tw, k.tw_z);
     F::template first<true>(buf, t, v);
     F::template finish<true>(TwRows<N>{tw}, buf, t, v);
     {
