@@ -63,13 +63,13 @@ __host__ __device__ constexpr int pair_slots(int n)
     return n + (pair_pad(n, false) > pair_pad(n, true) ? pair_pad(n, false) : pair_pad(n, true));
 }
 
-// Pairs on neighbouring lanes (Q = 2): eight butterflies of each make up a
-// 16-lane access, so the pairs' slots start half of the banks apart.
+// Pairs on neighbouring lanes: 16 / Q butterflies of each of the Q pairs make up
+// a 16-lane access, so the pairs' slots start 16 / Q banks apart.
 __host__ __device__ constexpr int pair_slots_q(int n, int q)
 {
     int s = pair_slots(n);
-    if (q == 2)
-        while (s % 16 != 8) ++s;
+    if (q > 1)
+        while (s % 16 != 16 / q) ++s;
     return s;
 }
 

@@ -20,16 +20,17 @@ __constant__ int c_fwd[9] = {1, 1, 1, 0, 0, 0, 0, 0, 0};
 // G indices that go through the x and y passes (all but kGz)
 __constant__ int c_gxy[kNumGxy] = {0, 1, 2, 3, 5, 6, 8, 9, 11, 12, 13, 14, 15, 17, 18, 19, 20, 21, 23, 24, 26};
 
+#if QVTI_PART == 0
 // ------------------------------------------------------------------ k_fz --
+// The runtime-length kernel (k_fp below is the compiled form).
 // R2C along z of vx, vy, vz.  Tile: one x, P consecutive y rows (P even);
 // rows (2q, 2q+1) share one complex transform.  Output H[f][kz][x][y].
-template <int N>
-__global__ void __launch_bounds__(kThreads) k_fz(KP k, int P_rt)
+__global__ void __launch_bounds__(kThreads) k_fz(KP k, int P)
 {
+    constexpr int N = 0;
     extern __shared__ float4 smem4[];
     float2* sm = reinterpret_cast<float2*>(smem4);
-    const int P = N > 0 ? 16 : P_rt;
-    const int n = N > 0 ? N : k.nz, Qp = P / 2, ps = n + n / 16;
+    const int n = k.nz, Qp = P / 2, ps = n + n / 16;
     float2* tw = sm;
     float2* A = tw + n;
     float2* B = A + Qp * ps;
@@ -53,6 +54,68 @@ __global__ void __launch_bounds__(kThreads) k_fz(KP k, int P_rt)
         const float2 z = Z[q * ps + kz];
         const float2 zm = cconj(Z[q * ps + (kz ? n - kz : 0)]);
         H[spec(k, kz, x, y0 + p)] = (p & 1) ? unpack_b(z, zm) : unpack_a(z, zm);
+    }
+}
+#endif  // QVTI_PART == 0
+
+// ------------------------------------------------------------------ k_fp --
+// Compiled form of k_fz: 16 rows as four packed pairs, rows 0 + 2 i and 1 + 3 i
+// of a quad in each (fft_pair.cuh), the four quads of a butterfly on
+// neighbouring lanes; the unpacking reads the planes pair-fastest, so four
+// lanes write one 128-byte line of the spectrum (96 against 118 us for k_fz at
+// 256^3, 27 against 40 at 150^3, 359 against 439 at 512x512x256).
+constexpr int kFpPairs = 4;
+constexpr int fp_threads(int n) { return warps_up(kFpPairs * pair_tasks(n)); }
+constexpr size_t fp_smem(int n) { return 16 * ((size_t)kFpPairs * pair_slots_q(n, kFpPairs) + tw_rows_size(n)); }
+constexpr int fp_blocks(int n)
+{
+    const int warps = fp_threads(n) / 32;
+    int b = 65536 / ((pair_rmax(n) >= 10 ? 128 : 80) * fp_threads(n));
+    while (b > 1 && b * warps % 4) --b;
+    return b < 1 ? 1 : b;
+}
+
+template <int N>
+__global__ void __launch_bounds__(fp_threads(N), fp_blocks(N)) k_fp(KP k)
+{
+    using F = PairFFT<N, kFpPairs, false, false, kFpPairs>;
+    constexpr int NT = fp_threads(N), RM = pair_rmax(N), R0 = F::R0, RL = F::RL;
+    extern __shared__ float4 smem4[];
+    f2* buf = reinterpret_cast<f2*>(smem4);
+    float4* tw = smem4 + F::PLANE;
+    const int t = threadIdx.x, x = blockIdx.y, y0 = blockIdx.x * 4 * kFpPairs;
+    c2 v[RM];
+    int p, j;
+    if (F::template task<0>(t, p, j)) {
+        const int left = k.ny - y0 - 4 * p;  // rows of the quad inside the grid: 4 or more, 2, none
+        const float* s = k.v[blockIdx.z] + cell(k, x, y0 + 4 * p, j);
+#pragma unroll
+        for (int r = 0; r < R0; ++r) {
+            const float* a = s + r * (N / R0);
+            v[r] = c2{left > 0 ? pack2(a[0], a[N]) : pack2(0.f, 0.f), left > 2 ? pack2(a[2 * N], a[3 * N]) : pack2(0.f, 0.f)};
+        }
+    }
+    TwRows<N>::template fill<NT>(tw, k.tw_z);
+    F::template first<false>(buf, t, v);
+    F::template finish<false>(TwRows<N>{tw}, buf, t, v);
+    constexpr int D = F::template dist<F::NST - 1>();
+    if (F::template task<F::NST - 1>(t, p, j)) {
+#pragma unroll
+        for (int r = 0; r < RL; ++r) F::st(buf + F::slot(p, j) + r * D, v[r]);
+    }
+    __syncthreads();
+    float2* H = k.H[blockIdx.z];
+    const f2 half = pack2(0.5f, 0.5f);
+    for (int w = t; w < kFpPairs * (N / 2 + 1); w += NT) {
+        const int q = w % kFpPairs, kz = (unsigned)w / kFpPairs, y = y0 + 4 * q;
+        if (y >= k.ny) continue;
+        const c2 z = F::ld(buf + F::slot(q, kz)), m = F::ld(buf + F::slot(q, kz ? N - kz : 0));
+        // rows 0, 1: (Z + conj Z(-k)) / 2; rows 2, 3: (Z - conj Z(-k)) / 2i
+        const float2 ar = unpack2((z.x + m.x) * half), ai = unpack2((z.y - m.y) * half);
+        const float2 br = unpack2((z.y + m.y) * half), bi = unpack2((m.x - z.x) * half);
+        float4* to = reinterpret_cast<float4*>(H + spec(k, kz, x, y));
+        to[0] = make_float4(ar.x, ai.x, ar.y, ai.y);
+        if (y + 2 < k.ny) to[1] = make_float4(br.x, bi.x, br.y, bi.y);
     }
 }
 
@@ -419,7 +482,8 @@ template <>
 bool fz_launch<QVTI_PART>(const KP& k, int P, int ncomp, cudaStream_t st)
 {
     return dispatch_len(k.nz, [&](auto NN) {
-        k_fz<decltype(NN)::value><<<dim3(cdiv(k.ny, P), k.nx, ncomp), kThreads, smem_fz(k, P), st>>>(k, P);
+        constexpr int N = decltype(NN)::value;
+        k_fp<N><<<dim3(cdiv(k.ny, P), k.nx, ncomp), fp_threads(N), fp_smem(N), st>>>(k);
     });
 }
 template <>
@@ -446,7 +510,7 @@ bool sp_configure<QVTI_PART>(SmemLimit& lim)
     for (int n : kMyLengths)
         dispatch_len(n, [&](auto NN) {
             constexpr int N = decltype(NN)::value;
-            lim.set((const void*)k_fz<N>);
+            lim.set((const void*)k_fp<N>);
             lim.set((const void*)k_cp<N, false>);
             lim.set((const void*)k_cp<N, true>);
             if constexpr (N >= kMinLong) lim.set((const void*)k_mp<N>);
@@ -455,7 +519,11 @@ bool sp_configure<QVTI_PART>(SmemLimit& lim)
 }
 
 #if QVTI_PART == 0
-size_t smem_fz(const KP& k, int P) { return sizeof(float2) * (k.nz + 2 * (P / 2) * (k.nz + k.nz / 16)); }
+size_t smem_fz(const KP& k, int P, bool rt)
+{
+    if (!rt) return fp_smem(k.nz);
+    return sizeof(float2) * (k.nz + 2 * (P / 2) * (k.nz + k.nz / 16));
+}
 size_t smem_cy(const KP& k, int L, bool ydv, bool rt)
 {
     if (!rt) return cp_smem(k.ny);
@@ -470,7 +538,7 @@ size_t smem_mx(const KP& k, int P, bool rt)
 
 void launch_fz(const KP& k, int P, bool rt, int ncomp, cudaStream_t st)
 {
-    if (rt) k_fz<0><<<dim3(cdiv(k.ny, P), k.nx, ncomp), rt_threads(k.pz, P / 2), smem_fz(k, P), st>>>(k, P);
+    if (rt) k_fz<<<dim3(cdiv(k.ny, P), k.nx, ncomp), rt_threads(k.pz, P / 2), smem_fz(k, P, true), st>>>(k, P);
     else (void)QVTI_CALL_PARTS(fz_launch, k, P, ncomp, st);
 }
 
@@ -493,7 +561,7 @@ void launch_mx(const KP& k, int P, bool rt, int kz0, int nb, cudaStream_t st)
 cudaError_t configure_spectral()
 {
     SmemLimit lim;
-    lim.set((const void*)k_fz<0>);
+    lim.set((const void*)k_fz);
     lim.set((const void*)k_cy<false>);
     lim.set((const void*)k_cy<true>);
     lim.set((const void*)k_mx);

@@ -138,7 +138,7 @@ void launch_mx(const KP& k, int P, bool rt, int kz0, int nb, cudaStream_t st);
 void launch_sigma(const KP& k, int P, bool rt, cudaStream_t st);
 // Their dynamic shared memory (bytes).
 size_t smem_vyx(int n, int P, bool rt);
-size_t smem_fz(const KP& k, int P);
+size_t smem_fz(const KP& k, int P, bool rt);
 size_t smem_cy(const KP& k, int L, bool ydv, bool rt);
 size_t smem_mx(const KP& k, int P, bool rt);
 size_t smem_sigma(const KP& k, int P, bool rt);

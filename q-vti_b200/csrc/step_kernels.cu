@@ -378,7 +378,7 @@ size_t step_smem_bytes(const KP& k)
     const StepTiles T = step_tiles(k);
     size_t m = smem_vyx(k.ny, T.vy, T.rt[0]);
     m = std::max(m, smem_vyx(k.nx, T.vx, T.rt[1]));
-    m = std::max(m, smem_fz(k, T.fz));
+    m = std::max(m, smem_fz(k, T.fz, T.rt[2]));
     m = std::max(m, smem_cy(k, T.cy, true, T.rt[3]));
     m = std::max(m, smem_mx(k, T.mx, T.rt[4]));
     m = std::max(m, smem_sigma(k, T.sigma, T.rt[5]));
