@@ -382,6 +382,11 @@ size_t step_smem_bytes(const KP& k)
     m = std::max(m, smem_cy(k, T.cy, true, T.rt[3]));
     m = std::max(m, smem_mx(k, T.mx, T.rt[4]));
     m = std::max(m, smem_sigma(k, T.sigma, T.rt[5]));
+    // the grids and tiles that are supported at runtime z lengths are those of
+    // a layout with room for the z derivatives and their tables beside the fields
+    if (T.rt[5])
+        m = std::max(m, smem_sigma(k, T.sigma, true) + sizeof(float2) * 2 * k.nz +
+                            sizeof(float) * ((size_t)3 * T.sigma * (k.nz + 1) + 4 * k.nz + 4 * T.sigma));
     return m;
 }
 
