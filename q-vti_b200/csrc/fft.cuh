@@ -510,151 +510,3 @@ __device__ __forceinline__ float2 two_shift(float2 z, float2 zmc, float2 f, floa
 }
 
 }  // namespace qvti
-
-namespace qvti {
-
-// ------------------------------------------------- compile-time transforms --
-// The same Stockham sequence with the length, the radix plan, the tile width
-// and the block size known at compile time: every index division becomes a
-// shift or a multiply, every stage loop has a fixed trip count.  Used for the
-// common grid sizes; the runtime fft_run covers the rest.
-__host__ __device__ constexpr int ct_nst(int n) { return radix_seq(n).nst; }
-__host__ __device__ constexpr int ct_rad(int n, int stage) { return radix_seq(n).rad[stage]; }
-__host__ __device__ constexpr int ct_ns(int n, int stage)
-{
-    int p = 1;
-    for (int s = 0; s < stage; ++s) p *= ct_rad(n, s);
-    return p;
-}
-
-// Tile layouts in shared memory (element (p, i) of pencil p, index i):
-//   kLine     p (N + 1) + i                  line-major
-//   kPencil   p + (i + i/16) P               pencil-fastest, one pad row per 16
-//   kLinePad  p (N + N/16) + i + i/16        line-major, one pad per 16
-// The thread mapping follows the layout: pencil-fastest tiles put
-// consecutive pencils on consecutive lanes (for data whose pencils are
-// adjacent in memory), line-major ones consecutive indices (for data whose
-// transform axis is contiguous: a half warp then reads 16 consecutive points
-// of one line).  With radix-16 first and last stages both padded layouts are
-// free of bank conflicts.
-constexpr int kLine = 0, kPencil = 1, kLinePad = 2;
-
-// PRETW (two-stage transforms only): stage 0 multiplies its outputs by the
-// twiddles stage 1 would apply to them, so stage 1 starts its butterflies
-// straight from shared memory.  The products are the same, on the same
-// values; what changes is where they are computed: after stage 0's loads are
-// consumed, instead of with 16 values and 15 twiddles live in stage 1 (which
-// at 256 points spills under a 72-register cap).
-// ROLL: a stage of several butterfly rounds per thread (small radices, many
-// pencils) stays a loop instead of being unrolled, so the compiler does not
-// hoist every round's loads at once; for a kernel already near its register
-// cap that is the difference between spilling and not.
-template <int N, int P, int NT, int LY, bool PRETW = false, bool ROLL = false>
-struct FftCT {
-    static constexpr bool PF = LY == kPencil;
-    static constexpr int NST = ct_nst(N);
-    static constexpr int BUF = LY == kLine ? P * (N + 1) : P * (N + N / 16);  // float2 per buffer
-
-    static constexpr int PSTEP = LY == kPencil ? P : 1;  // distance of consecutive indices
-    static_assert(!PRETW || NST == 2, "stage-1 twiddles move into stage 0 only for two-stage transforms");
-
-    static __device__ __forceinline__ int at(int p, int i)
-    {
-        if constexpr (LY == kPencil) return p + (i + (i >> 4)) * P;
-        else if constexpr (LY == kLinePad) return p * (N + N / 16) + i + (i >> 4);
-        else return p * (N + 1) + i;
-    }
-
-    template <int S, bool INV, class Load, class Store>
-    static __device__ __forceinline__ void stage(const float2* __restrict__ tw, float2* A, float2* B, Load& load,
-                                                 Store& store)
-    {
-        constexpr int R = ct_rad(N, S), NS = ct_ns(N, S);
-        constexpr bool FIRST = S == 0, LAST = S == NST - 1;
-        constexpr int NR = N / R, TOTAL = P * NR, TWS = N / (NS * R);
-        const float2* src = ((S - 1) & 1) ? B : A;
-        float2* dst = (S & 1) ? B : A;
-        constexpr int ITER = (TOTAL + NT - 1) / NT;
-        constexpr int UNR = ROLL ? 1 : ITER;
-#pragma unroll(UNR)
-        for (int it = 0; it < ITER; ++it) {
-            const int t = threadIdx.x + it * NT;
-            if ((TOTAL % NT) != 0 && t >= TOTAL) break;
-            int p, j;
-            if (PF) { p = t % P; j = t / P; }
-            else    { j = t % NR; p = t / NR; }
-            const int jm = j % NS;
-            float2 v[R];
-            if constexpr (FIRST) {
-#pragma unroll
-                for (int r = 0; r < R; ++r) v[r] = load(p, j + r * NR);
-            } else if constexpr (LY != kLine && NR % 16 == 0) {
-                // idx = j + r NR: the pad row advances by NR/16 per r
-                const int b = at(p, j);
-#pragma unroll
-                for (int r = 0; r < R; ++r) v[r] = src[b + r * (NR + NR / 16) * PSTEP];
-            } else {
-#pragma unroll
-                for (int r = 0; r < R; ++r) v[r] = src[at(p, j + r * NR)];
-            }
-            if constexpr (!FIRST && !PRETW) {
-                if (jm) {
-#pragma unroll
-                    for (int r = 1; r < R; ++r) {
-                        const float2 w = tw[jm * r * TWS];
-                        v[r] = INV ? cmulc(v[r], w) : cmul(v[r], w);
-                    }
-                }
-            }
-            Dft<R>::template run<INV>(v);
-            if constexpr (PRETW && FIRST) {
-                // two stages (NS = 1 here, R0 = NS of stage 1, TWS of stage 1
-                // = 1): output r of butterfly j lands at index j R + r, which
-                // stage 1 reads as its butterfly r, element j, with twiddle
-                // w^(r j)
-                if (j) {
-#pragma unroll
-                    for (int r = 1; r < R; ++r) {
-                        const float2 w = tw[r * j];
-                        v[r] = INV ? cmulc(v[r], w) : cmul(v[r], w);
-                    }
-                }
-            }
-            const int base = (j - jm) * R + jm;
-            if constexpr (LAST) {
-#pragma unroll
-                for (int r = 0; r < R; ++r) store(p, base + r * NS, v[r]);
-            } else if constexpr (LY != kLine && NS % 16 == 0) {
-                // idx = base + r NS: the pad row advances by NS/16 per r
-                const int b = at(p, base);
-#pragma unroll
-                for (int r = 0; r < R; ++r) dst[b + r * (NS + NS / 16) * PSTEP] = v[r];
-            } else if constexpr (LY != kLine && 16 % (NS * R) == 0) {
-                // the R outputs lie in one aligned run of NS R <= 16 indices
-                // (base = m NS R + jm, jm < NS): one pad row for all of them
-                const int b = at(p, base);
-#pragma unroll
-                for (int r = 0; r < R; ++r) dst[b + r * NS * PSTEP] = v[r];
-            } else {
-#pragma unroll
-                for (int r = 0; r < R; ++r) dst[at(p, base + r * NS)] = v[r];
-            }
-        }
-        __syncthreads();
-        if constexpr (!LAST) stage<S + 1, INV>(tw, A, B, load, store);
-    }
-
-    // Stage 0 reads `load`, the last stage writes `store`; ends with
-    // __syncthreads().  Buffers: A always, B when NST > 2.
-    template <bool INV, class Load, class Store>
-    static __device__ __forceinline__ void run(const float2* __restrict__ tw, float2* A, float2* B, Load load,
-                                               Store store)
-    {
-        stage<0, INV>(tw, A, B, load, store);
-    }
-
-    // The buffer the last stage does not read.
-    static __device__ __forceinline__ float2* out_buf(float2* A, float2* B) { return ((NST - 1) & 1) ? B : A; }
-};
-
-}  // namespace qvti

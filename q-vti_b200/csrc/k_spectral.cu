@@ -27,7 +27,6 @@ __constant__ int c_gxy[kNumGxy] = {0, 1, 2, 3, 5, 6, 8, 9, 11, 12, 13, 14, 15, 1
 // rows (2q, 2q+1) share one complex transform.  Output H[f][kz][x][y].
 __global__ void __launch_bounds__(kThreads) k_fz(KP k, int P)
 {
-    constexpr int N = 0;
     extern __shared__ float4 smem4[];
     float2* sm = reinterpret_cast<float2*>(smem4);
     const int n = k.nz, Qp = P / 2, ps = n + n / 16;
@@ -39,14 +38,14 @@ __global__ void __launch_bounds__(kThreads) k_fz(KP k, int P)
     const int f = blockIdx.z, x = blockIdx.y, y0 = blockIdx.x * P;
     const int yv = min(P, k.ny - y0);  // rows of the tile inside the grid (even)
     const float* src = k.v[f];
-    float2* Z = out_any<N, 8, kThreads, kLinePad>(k.pz, A, B);
+    float2* Z = fft_out_buf(k.pz, A, B);
     auto load = [&](int q, int i) -> float2 {
         if (2 * q >= yv) return make_float2(0.f, 0.f);
         const int b = cell(k, x, y0 + 2 * q, i);
         return make_float2(src[b], src[b + n]);
     };
     auto store = [&](int q, int i, float2 v) { Z[q * ps + i] = v; };
-    fft_any<N, 8, kThreads, kLinePad, false>(k.pz, tw, A, B, Qp, ps, 1, load, store);
+    fft_rt<kLinePad, false>(k.pz, tw, A, B, Qp, ps, 1, load, store);
     float2* H = k.H[f];
     for (int t = threadIdx.x; t < k.nkz * P; t += blockDim.x) {
         const int p = t % P, kz = t / P, q = p >> 1;
@@ -133,7 +132,6 @@ constexpr int kCyThreads = 128;
 template <bool INV>
 __global__ void __launch_bounds__(kCyThreads) k_cy(KP k, int L, long long line0, long long line_end)
 {
-    constexpr int N = 0;
     extern __shared__ float4 smem4[];
     float2* sm = reinterpret_cast<float2*>(smem4);
     const int n = k.ny;
@@ -157,7 +155,7 @@ __global__ void __launch_bounds__(kCyThreads) k_cy(KP k, int L, long long line0,
         if (p < lv) dst[(long long)p * n + i] = v;
         if (ydv) C[p * n + i] = v;
     };
-    fft_any<N, 8, kCyThreads, kLinePad, INV>(k.py, tw, A, B, L, n + n / 16, 1, load, store);
+    fft_rt<kLinePad, INV>(k.py, tw, A, B, L, n + n / 16, 1, load, store);
     if constexpr (!INV) {
         if (ydv) {
             // the y derivative with the identity dispersion operator, scaled
@@ -171,7 +169,7 @@ __global__ void __launch_bounds__(kCyThreads) k_cy(KP k, int L, long long line0,
             auto store_d = [&](int p, int i, float2 v) {
                 if (p < lv) yd[(long long)p * n + i] = v;
             };
-            fft_any<N, 8, kCyThreads, kLinePad, true>(k.py, tw, A, B, L, n + n / 16, 1, load_d, store_d);
+            fft_rt<kLinePad, true>(k.py, tw, A, B, L, n + n / 16, 1, load_d, store_d);
         }
     }
 }
@@ -267,7 +265,6 @@ __global__ void __launch_bounds__(cp_threads(N), cp_blocks(N)) k_cp(KP k, long l
 // x-transformed on chip.  blockIdx.y + kz0 is the kz plane.
 __global__ void __launch_bounds__(kThreads) k_mx(KP k, int P, int kz0)
 {
-    constexpr int N = 0;
     extern __shared__ float4 smem4[];
     float2* sm = reinterpret_cast<float2*>(smem4);
     const int n = k.nx;
@@ -303,7 +300,7 @@ __global__ void __launch_bounds__(kThreads) k_mx(KP k, int P, int kz0)
         const float2* H = k.Hy[c];
         auto load = [&](int p, int i) -> float2 { return p < yv ? H[spec(k, kz, i, y0 + p)] : make_float2(0.f, 0.f); };
         auto store = [&](int p, int i, float2 v) { V[i * P + p] = v; };
-        fft_any<N, 16, kThreads, kPencil, false>(k.px, tw, A, B, P, 1, P, load, store);
+        fft_rt<kPencil, false>(k.px, tw, A, B, P, 1, P, load, store);
     }
 
     const float kzv = k.kz[kz];
@@ -333,7 +330,7 @@ __global__ void __launch_bounds__(kThreads) k_mx(KP k, int P, int kz0)
             auto store = [&](int p, int i, float2 v) {
                 if (p < yv) G[spec(k, kz, i, y0 + p)] = v;
             };
-            fft_any<N, 16, kThreads, kPencil, true>(k.px, tw, A, B, P, 1, P, load, store);
+            fft_rt<kPencil, true>(k.px, tw, A, B, P, 1, P, load, store);
         }
     }
 }

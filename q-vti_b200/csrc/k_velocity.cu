@@ -17,7 +17,6 @@ namespace {
 // needs before storing anything (no store can delay a later load).
 __global__ void __launch_bounds__(kThreads) k_vy(KP k, int P)
 {
-    constexpr int N = 0;
     extern __shared__ float4 smem4[];
     float2* sm = reinterpret_cast<float2*>(smem4);
     const int n = k.ny, ny = n, pml = k.pml;
@@ -45,17 +44,17 @@ __global__ void __launch_bounds__(kThreads) k_vy(KP k, int P)
 
     // pass 1: sxy + i syy -> dy+ sxy (vx), dy- syy (vy)
     if (blockIdx.z == 0) {
-        float2* Zf = out_any<N, 16, kThreads, kPencil>(k.py, A, B);
+        float2* Zf = fft_out_buf(k.py, A, B);
         auto load = [&](int p, int i) -> float2 {
             if (p >= zv) return make_float2(0.f, 0.f);
             const int ip = cell(k, x, i, z0 + p);
             return make_float2(sxy[ip], syy[ip]);
         };
         auto store = [&](int p, int i, float2 v) { Zf[i * P + p] = v; };
-        fft_any<N, 16, kThreads, kPencil, false>(k.py, tw, A, B, P, 1, P, load, store);
+        fft_rt<kPencil, false>(k.py, tw, A, B, P, 1, P, load, store);
         float2* X1 = Zf == A ? B : A;
         // [2][n][P] in the buffer the last stage does not read
-        float* D = reinterpret_cast<float*>(out_any<N, 16, kThreads, kPencil>(k.py, X1, Zf));
+        float* D = reinterpret_cast<float*>(fft_out_buf(k.py, X1, Zf));
         auto load_i = [&](int p, int i) -> float2 {
             const int im = i ? n - i : 0;
             return two_shift(Zf[i * P + p], cconj(Zf[im * P + p]), cscale(tF[i], inv_n), 1.0f);
@@ -64,7 +63,7 @@ __global__ void __launch_bounds__(kThreads) k_vy(KP k, int P)
             D[i * P + p] = v.x;
             D[(n + i) * P + p] = v.y;
         };
-        fft_any<N, 16, kThreads, kPencil, true>(k.py, tw, X1, Zf, P, 1, P, load_i, store_i);
+        fft_rt<kPencil, true>(k.py, tw, X1, Zf, P, 1, P, load_i, store_i);
         // kEpi cells per thread and trip: all their loads are in flight at once
         for (int t0 = threadIdx.x; t0 < n * P; t0 += kEpi * blockDim.x) {
             int ipu[kEpi], iu[kEpi], pu[kEpi], isu[kEpi];
@@ -108,22 +107,22 @@ __global__ void __launch_bounds__(kThreads) k_vy(KP k, int P)
     // pass 2: syz, pencils (2q, 2q+1) -> dy+ syz (vz)
     {
         const int Qp = P / 2;
-        float2* Zf = out_any<N, 8, kThreads, kPencil>(k.py, A, B);
+        float2* Zf = fft_out_buf(k.py, A, B);
         auto load = [&](int q, int i) -> float2 {
             if (2 * q >= zv) return make_float2(0.f, 0.f);
             const int ip = cell(k, x, i, z0 + 2 * q);
             return *reinterpret_cast<const float2*>(syz + ip);
         };
         auto store = [&](int q, int i, float2 v) { Zf[i * Qp + q] = v; };
-        fft_any<N, 8, kThreads, kPencil, false>(k.py, tw, A, B, Qp, 1, Qp, load, store);
+        fft_rt<kPencil, false>(k.py, tw, A, B, Qp, 1, Qp, load, store);
         float2* X1 = Zf == A ? B : A;
-        float* D = reinterpret_cast<float*>(out_any<N, 8, kThreads, kPencil>(k.py, X1, Zf));  // [n][P]
+        float* D = reinterpret_cast<float*>(fft_out_buf(k.py, X1, Zf));  // [n][P]
         auto load_i = [&](int q, int i) -> float2 { return cmul(Zf[i * Qp + q], cscale(tF[i], inv_n)); };
         auto store_i = [&](int q, int i, float2 v) {
             D[i * P + 2 * q] = v.x;
             D[i * P + 2 * q + 1] = v.y;
         };
-        fft_any<N, 8, kThreads, kPencil, true>(k.py, tw, X1, Zf, Qp, 1, Qp, load_i, store_i);
+        fft_rt<kPencil, true>(k.py, tw, X1, Zf, Qp, 1, Qp, load_i, store_i);
         for (int t0 = threadIdx.x; t0 < n * P; t0 += kEpi * blockDim.x) {
             int ipu[kEpi], iu[kEpi], pu[kEpi], isu[kEpi];
             bool ok[kEpi], slab[kEpi];
@@ -164,7 +163,6 @@ __global__ void __launch_bounds__(kThreads) k_vy(KP k, int P)
 // park-then-epilogue structure as k_vy.
 __global__ void __launch_bounds__(kThreads) k_vx(KP k, int P)
 {
-    constexpr int N = 0;
     extern __shared__ float4 smem4[];
     float2* sm = reinterpret_cast<float2*>(smem4);
     const int n = k.nx, nx = n, pml = k.pml;
@@ -197,16 +195,16 @@ __global__ void __launch_bounds__(kThreads) k_vx(KP k, int P)
 
     // pass 1: sxx + i sxy -> dx- sxx (vx), dx+ sxy (vy)
     if (blockIdx.z == 0) {
-        float2* Zf = out_any<N, 16, kThreads, kPencil>(k.px, A, B);
+        float2* Zf = fft_out_buf(k.px, A, B);
         auto load = [&](int p, int i) -> float2 {
             if (p >= zv) return make_float2(0.f, 0.f);
             const int ip = cell(k, i, y, z0 + p);
             return make_float2(sxx[ip], sxy[ip]);
         };
         auto store = [&](int p, int i, float2 v) { Zf[i * P + p] = v; };
-        fft_any<N, 16, kThreads, kPencil, false>(k.px, tw, A, B, P, 1, P, load, store);
+        fft_rt<kPencil, false>(k.px, tw, A, B, P, 1, P, load, store);
         float2* X1 = Zf == A ? B : A;
-        float* D = reinterpret_cast<float*>(out_any<N, 16, kThreads, kPencil>(k.px, X1, Zf));  // [2][n][P]
+        float* D = reinterpret_cast<float*>(fft_out_buf(k.px, X1, Zf));  // [2][n][P]
         auto load_i = [&](int p, int i) -> float2 {
             const int im = i ? n - i : 0;
             return two_shift(Zf[i * P + p], cconj(Zf[im * P + p]), cscale(tF[i], inv_n), -1.0f);
@@ -215,7 +213,7 @@ __global__ void __launch_bounds__(kThreads) k_vx(KP k, int P)
             D[i * P + p] = v.x;
             D[(n + i) * P + p] = v.y;
         };
-        fft_any<N, 16, kThreads, kPencil, true>(k.px, tw, X1, Zf, P, 1, P, load_i, store_i);
+        fft_rt<kPencil, true>(k.px, tw, X1, Zf, P, 1, P, load_i, store_i);
         for (int t0 = threadIdx.x; t0 < n * P; t0 += kEpi * blockDim.x) {
             int ipu[kEpi], iu[kEpi], pu[kEpi], isu[kEpi];
             bool ok[kEpi], slab[kEpi];
@@ -262,22 +260,22 @@ __global__ void __launch_bounds__(kThreads) k_vx(KP k, int P)
     // pass 2: sxz pencils (2q, 2q+1) -> dx+ sxz (vz)
     {
         const int Qp = P / 2;
-        float2* Zf = out_any<N, 8, kThreads, kPencil>(k.px, A, B);
+        float2* Zf = fft_out_buf(k.px, A, B);
         auto load = [&](int q, int i) -> float2 {
             if (2 * q >= zv) return make_float2(0.f, 0.f);
             const int ip = cell(k, i, y, z0 + 2 * q);
             return *reinterpret_cast<const float2*>(sxz + ip);
         };
         auto store = [&](int q, int i, float2 v) { Zf[i * Qp + q] = v; };
-        fft_any<N, 8, kThreads, kPencil, false>(k.px, tw, A, B, Qp, 1, Qp, load, store);
+        fft_rt<kPencil, false>(k.px, tw, A, B, Qp, 1, Qp, load, store);
         float2* X1 = Zf == A ? B : A;
-        float* D = reinterpret_cast<float*>(out_any<N, 8, kThreads, kPencil>(k.px, X1, Zf));  // [n][P]
+        float* D = reinterpret_cast<float*>(fft_out_buf(k.px, X1, Zf));  // [n][P]
         auto load_i = [&](int q, int i) -> float2 { return cmul(Zf[i * Qp + q], cscale(tF[i], inv_n)); };
         auto store_i = [&](int q, int i, float2 v) {
             D[i * P + 2 * q] = v.x;
             D[i * P + 2 * q + 1] = v.y;
         };
-        fft_any<N, 8, kThreads, kPencil, true>(k.px, tw, X1, Zf, Qp, 1, Qp, load_i, store_i);
+        fft_rt<kPencil, true>(k.px, tw, X1, Zf, Qp, 1, Qp, load_i, store_i);
         for (int t0 = threadIdx.x; t0 < n * P; t0 += kEpi * blockDim.x) {
             int ipu[kEpi], iu[kEpi], pu[kEpi], isu[kEpi];
             bool ok[kEpi], slab[kEpi];

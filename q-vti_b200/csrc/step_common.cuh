@@ -26,23 +26,15 @@ __device__ __forceinline__ void load_table(float2* s, const float2* g, int n)
     for (int i = threadIdx.x; i < n; i += blockDim.x) s[i] = g[i];
 }
 
-// A transform of the tile through the compile-time path (N > 0: length N, PC
-// pencils, NT threads) or the runtime one (N == 0: plan pl, prt pencils,
-// layout ps_rt/is_rt).  LY is the shared-memory layout (kLine, kPencil,
-// kLinePad); the padded layouts carry one padding row every 16 indices in
-// both paths.
-template <int N, int PC, int NT, int LY, bool INV, bool ROLL = false, class Load, class Store>
-__device__ __forceinline__ void fft_any(const FftPlan& pl, const float2* tw, float2* A, float2* B, int prt, int ps_rt,
-                                        int is_rt, Load load, Store store)
+// Tile layouts of the runtime kernels in shared memory: pencil-fastest (for
+// pencils that are adjacent in memory) or line-major, both with one padding row
+// every 16 indices.
+constexpr int kPencil = 1, kLinePad = 2;
+template <int LY, bool INV, class Load, class Store>
+__device__ __forceinline__ void fft_rt(const FftPlan& pl, const float2* tw, float2* A, float2* B, int pencils, int ps,
+                                       int is, Load load, Store store)
 {
-    if constexpr (N > 0) FftCT<N, PC, NT, LY, false, ROLL>::template run<INV>(tw, A, B, load, store);
-    else fft_run<LY == kPencil, INV>(pl, tw, A, B, prt, ps_rt, is_rt, load, store, LY == kLine ? 0 : 4);
-}
-template <int N, int PC, int NT, int LY>
-__device__ __forceinline__ float2* out_any(const FftPlan& pl, float2* A, float2* B)
-{
-    if constexpr (N > 0) return FftCT<N, PC, NT, LY>::out_buf(A, B);
-    else return fft_out_buf(pl, A, B);
+    fft_run<LY == kPencil, INV>(pl, tw, A, B, pencils, ps, is, load, store, 4);
 }
 
 // Transform lengths with a compile-time path: the 5-smooth lengths the
