@@ -59,11 +59,9 @@ bool smooth(int n)
 // shared-memory sizes derived from them).
 bool make_plan(int n, FftPlan* p)
 {
-    const RadixSeq q = radix_seq(n);
     p->n = n;
-    p->nst = q.nst;
-    for (int s = 0; s < kMaxStages; ++s) p->rad[s] = q.rad[s];
-    return q.nst >= 2;
+    p->q = radix_seq(n);
+    return p->q.nst >= 2;
 }
 
 // FP64 construction of the 1D tables of one axis on the GPU:

@@ -3,7 +3,7 @@
 // The spectral-derivative engine replaces the reference's 63 cuFFT C2C calls
 // per step (cuviscoelas_3D.cu:1272-1562) with pencil kernels that transform a
 // tile of P pencils of one axis on chip.  A transform of length n = prod(rad)
-// runs as a Stockham autosort sequence of stages of radix up to 16:
+// runs as a Stockham autosort sequence of stages of up to 16 points:
 //
 //   * stage 0 reads its inputs through a caller-supplied `load(p, i)` functor
 //     (straight from global memory, or from shared memory with a k-space
@@ -27,39 +27,51 @@ namespace qvti {
 
 constexpr int kMaxStages = 4;
 
-struct FftPlan {
-    int n;                   // transform length
-    int nst;                 // number of stages (>= 2)
-    int rad[kMaxStages];     // radix of each stage, first stage first
-};
-
 // Radix plan of a length, shared by the host, the runtime kernels and the
-// compiled ones: the fewest stages of radices up to 16 (each stage is one
-// exchange through shared memory and a barrier or two, whatever its radix:
-// 96 = 12 8 instead of 16 2 3, 150 = 15 10 instead of 2 3 5 5), and among
-// those the plan whose largest radix is smallest (512 = 8 8 8, not 16 16 2:
-// a stage's task count is N / radix, so equal radices keep every thread busy
-// in every stage), larger radices first.
-__host__ __device__ constexpr bool radix_ok(int r)
-{
-    return (r >= 2 && r <= 10) || r == 12 || r == 14 || r == 15 || r == 16;
-}
+// compiled ones.  The arithmetic is that of the elementary radices 16, 8, 4, 2,
+// 3, 5, 7 in this order (16 itself: 4 4); two neighbouring ones whose product is
+// at most 16 run as ONE stage, the second on the first's outputs in the same
+// registers (a then b; b = 1: a alone).  A stage is one exchange through shared
+// memory and a barrier or two, whatever its radix, so 96 = 16 (2 3) is two
+// stages; the values are those of the three separate ones.
 struct RadixSeq {
     int nst;
-    int rad[4];
+    int a[kMaxStages], b[kMaxStages];
+    int radices;  // elementary ones
+    constexpr int rad(int s) const { return a[s] * b[s]; }
 };
+__host__ __device__ constexpr bool radix_pair(int a, int b)
+{
+    return (a == 2 && (b == 3 || b == 5 || b == 7)) || (a == 4 && b == 3) || (a == 3 && (b == 3 || b == 5));
+}
 __host__ __device__ constexpr RadixSeq radix_seq(int n)
 {
-    RadixSeq best{0, {1, 1, 1, 1}};
-    for (int a = 2; a <= 16 && !best.nst; ++a)  // two stages a >= b
-        if (radix_ok(a) && n % a == 0 && n / a <= a && n / a >= 2 && radix_ok(n / a)) best = RadixSeq{2, {a, n / a, 1, 1}};
-    for (int a = 2; a <= 16 && !best.nst; ++a)  // three, a >= b >= c, b smallest
-        if (radix_ok(a) && n % a == 0)
-            for (int b = 2; b <= a && !best.nst; ++b)
-                if (radix_ok(b) && (n / a) % b == 0 && n / a / b <= b && n / a / b >= 2 && radix_ok(n / a / b))
-                    best = RadixSeq{3, {a, b, n / a / b, 1}};
-    return best;
+    int el[12] = {}, ne = 0, m = n;
+    const int order[7] = {16, 8, 4, 2, 3, 5, 7};
+    if (n == 16) {
+        el[0] = el[1] = 4;
+        ne = 2;
+        m = 1;
+    }
+    for (int i = 0; i < 7; ++i)
+        while (m % order[i] == 0 && ne < 12) {
+            el[ne++] = order[i];
+            m /= order[i];
+        }
+    RadixSeq q{0, {1, 1, 1, 1}, {1, 1, 1, 1}, ne};
+    if (m != 1 || ne < 2) return q;
+    for (int i = 0; i < ne; ++q.nst) {
+        if (q.nst == kMaxStages) return RadixSeq{0, {1, 1, 1, 1}, {1, 1, 1, 1}, ne};
+        q.a[q.nst] = el[i++];
+        if (i < ne && radix_pair(q.a[q.nst], el[i])) q.b[q.nst] = el[i++];
+    }
+    return q;
 }
+
+struct FftPlan {
+    int n;      // transform length
+    RadixSeq q;
+};
 
 // Two floats in one 64-bit register pair: sm_100a's packed FP32 instructions
 // do the operation on both in one issue slot.
@@ -137,13 +149,21 @@ __device__ __forceinline__ C cadd_rot(C a, C b)
 }
 template <bool INV, class C>
 __device__ __forceinline__ C csub_rot(C a, C b) { return cadd_rot<!INV>(a, b); }
+// Complex products.  The rounding of each is fixed here, which product of a sum
+// is rounded before the fused operation included: the scalar and the packed form
+// agree bit for bit, whatever the compiler contracts elsewhere.
 __device__ __forceinline__ float2 cmul(float2 a, float2 b)
 {
-    return make_float2(a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x);
+    return make_float2(fmaf(a.x, b.x, -(a.y * b.y)), fmaf(a.x, b.y, a.y * b.x));
+}
+// a times a multiplier m: the other product of the imaginary part first
+__device__ __forceinline__ float2 cmul_m(float2 a, float2 m)
+{
+    return make_float2(fmaf(a.x, m.x, -(a.y * m.y)), fmaf(a.y, m.x, a.x * m.y));
 }
 __device__ __forceinline__ float2 cmulc(float2 a, float2 b)  // a * conj(b)
 {
-    return make_float2(a.x * b.x + a.y * b.y, a.y * b.x - a.x * b.y);
+    return make_float2(fmaf(a.x, b.x, a.y * b.y), fmaf(a.y, b.x, -(a.x * b.y)));
 }
 // a times w (INV: conj(w)), w the same for both of a pair: (wx, wx), (wy, wy)
 template <bool INV>
@@ -151,29 +171,25 @@ __device__ __forceinline__ c2 cmul_tw(c2 a, f2 wx, f2 wy)
 {
     const f2 n = neg_(wy);
     c2 r;
-    r.x = fma_(a.y, INV ? wy : n, a.x * wx);
-    r.y = fma_(a.x, INV ? n : wy, a.y * wx);
+    r.x = fma_(a.x, wx, a.y * (INV ? wy : n));
+    r.y = INV ? fma_(a.y, wx, a.x * n) : fma_(a.x, wy, a.y * wx);
     return r;
 }
+__device__ __forceinline__ c2 cmul_m(c2 a, f2 mx, f2 my)
+{
+    c2 r;
+    r.x = fma_(a.x, mx, a.y * neg_(my));
+    r.y = fma_(a.y, mx, a.x * my);
+    return r;
+}
+template <bool INV>
+__device__ __forceinline__ float2 cmul_tw(float2 a, float2 w) { return INV ? cmulc(a, w) : cmul(a, w); }
 __device__ __forceinline__ float2 cscale(float2 a, float s) { return make_float2(a.x * s, a.y * s); }
 __device__ __forceinline__ float2 cconj(float2 a) { return make_float2(a.x, -a.y); }
-// a times cos - i sin (forward) or its conjugate (inverse), compile-time values
-template <bool INV, class C>
-__device__ __forceinline__ C cmul_cs(C a, float c, float s)
-{
-    if (INV) s = -s;
-    return cmake<C>(fmac_(a.x, c, scale_(a.y, s)), fmac_(a.y, c, scale_(a.x, -s)));
-}
 
 // ---------------------------------------------------------------- radix DFTs
 template <int R>
 struct Dft;
-
-template <>
-struct Dft<1> {
-    template <bool INV, class C>
-    static __device__ __forceinline__ void run(C*) {}
-};
 
 template <>
 struct Dft<2> {
@@ -213,21 +229,18 @@ struct Dft<8> {
         Dft<4>::run<INV>(o);
         // o[k] *= W8^k  (W8 = e^{-i pi/4} forward, conjugate inverse)
         const C r1 = cadd_rot<INV>(o[1], o[1]), r3 = csub_rot<INV>(o[3], o[3]);  // (1 -+ i) o1, (1 +- i) o3
-        const C t1 = cmake<C>(scale_(r1.x, c), scale_(r1.y, c));
-        const C t3 = cmake<C>(scale_(r3.x, c), scale_(r3.y, c));  // minus W8^3 o3
         v[0] = cadd(e[0], o[0]);
         v[4] = csub(e[0], o[0]);
-        v[1] = cadd(e[1], t1);
-        v[5] = csub(e[1], t1);
+        v[1] = cmake<C>(fmac_(r1.x, c, e[1].x), fmac_(r1.y, c, e[1].y));
+        v[5] = cmake<C>(fmac_(r1.x, -c, e[1].x), fmac_(r1.y, -c, e[1].y));
         v[2] = cadd_rot<INV>(e[2], o[2]);
         v[6] = csub_rot<INV>(e[2], o[2]);
-        v[3] = csub(e[3], t3);
-        v[7] = cadd(e[3], t3);
+        v[3] = cmake<C>(fmac_(r3.x, -c, e[3].x), fmac_(r3.y, -c, e[3].y));  // W8^3 o3 = -c r3
+        v[7] = cmake<C>(fmac_(r3.x, c, e[3].x), fmac_(r3.y, c, e[3].y));
     }
 };
 
-// Odd radices 3, 5, 7: the sums t_h = v[h] + v[R-h] carry the cosines, the
-// differences d_h the sines; outputs h and R-h share both products.
+// Odd radices 3, 5, 7: direct DFT.
 template <int R>
 __device__ constexpr float odd_cos(int k)
 {
@@ -235,8 +248,8 @@ __device__ constexpr float odd_cos(int k)
     if (2 * k > R) k = R - k;
     if (k == 0) return 1.f;
     if (R == 3) return -0.5f;
-    if (R == 5) return k == 1 ? 0.30901699437494742f : -0.80901699437494742f;
-    return k == 1 ? 0.62348980185873353f : k == 2 ? -0.22252093395631440f : -0.90096886790241913f;
+    if (R == 5) return k == 1 ? 0.309016994f : -0.809016994f;
+    return k == 1 ? 0.623489802f : k == 2 ? -0.222520934f : -0.900968868f;
 }
 template <int R>
 __device__ constexpr float odd_sin(int k)
@@ -245,9 +258,9 @@ __device__ constexpr float odd_sin(int k)
     const float sg = 2 * k > R ? -1.f : 1.f;
     if (2 * k > R) k = R - k;
     if (k == 0) return 0.f;
-    if (R == 3) return sg * 0.86602540378443865f;
-    if (R == 5) return sg * (k == 1 ? 0.95105651629515357f : 0.58778525229247313f);
-    return sg * (k == 1 ? 0.78183148246802981f : k == 2 ? 0.97492791218182361f : 0.43388373911755812f);
+    if (R == 3) return sg * 0.866025404f;
+    if (R == 5) return sg * (k == 1 ? 0.951056516f : 0.587785252f);
+    return sg * (k == 1 ? 0.781831482f : k == 2 ? 0.974927912f : 0.433883739f);
 }
 
 template <int R>
@@ -255,29 +268,21 @@ struct DftOdd {
     template <bool INV, class C>
     static __device__ __forceinline__ void run(C* v)
     {
-        constexpr int H = (R - 1) / 2;
-        C t[H], d[H];
+        C o[R];
+        o[0] = v[0];
 #pragma unroll
-        for (int h = 0; h < H; ++h) {
-            t[h] = cadd(v[h + 1], v[R - 1 - h]);
-            d[h] = csub(v[h + 1], v[R - 1 - h]);
+        for (int r = 1; r < R; ++r) o[0] = cadd(o[0], v[r]);
+#pragma unroll
+        for (int q = 1; q < R; ++q) {
+            o[q] = v[0];
+#pragma unroll
+            for (int r = 1; r < R; ++r) {
+                const float c = odd_cos<R>(q * r), s = INV ? odd_sin<R>(q * r) : -odd_sin<R>(q * r);
+                o[q] = cmake<C>(o[q].x + fmac_(v[r].x, c, scale_(v[r].y, -s)), o[q].y + fmac_(v[r].y, c, scale_(v[r].x, s)));
+            }
         }
-        const C v0 = v[0];
 #pragma unroll
-        for (int h = 0; h < H; ++h) v[0] = cadd(v[0], t[h]);
-#pragma unroll
-        for (int q = 1; q <= H; ++q) {
-            C m = v0;
-            C s = cmake<C>(scale_(d[0].x, odd_sin<R>(q)), scale_(d[0].y, odd_sin<R>(q)));
-#pragma unroll
-            for (int h = 1; h <= H; ++h)
-                m = cmake<C>(fmac_(t[h - 1].x, odd_cos<R>(q * h), m.x), fmac_(t[h - 1].y, odd_cos<R>(q * h), m.y));
-#pragma unroll
-            for (int h = 2; h <= H; ++h)
-                s = cmake<C>(fmac_(d[h - 1].x, odd_sin<R>(q * h), s.x), fmac_(d[h - 1].y, odd_sin<R>(q * h), s.y));
-            v[q] = cadd_rot<INV>(m, s);
-            v[R - q] = csub_rot<INV>(m, s);
-        }
+        for (int q = 0; q < R; ++q) v[q] = o[q];
     }
 };
 template <>
@@ -287,112 +292,69 @@ struct Dft<5> : DftOdd<5> {};
 template <>
 struct Dft<7> : DftOdd<7> {};
 
-// Radix A B with A and B coprime as A x B without twiddles (the prime-factor
-// map: input B n1 + A n2, output the k with k = k1 mod A, k = k2 mod B).
-// Inverse of a modulo m.
-__host__ __device__ constexpr int inv_mod(int a, int m)
+// Radix 16 in registers as 4 x 4: DFT-4 over n2 of v[n1 + 4 n2], twiddle
+// W16^{n1 k2}, DFT-4 over n1; output X[k2 + 4 k1].
+template <bool INV, class C>
+__device__ __forceinline__ C w16(C a, int e)  // e = 1, 2, 3, 6, 9
 {
-    for (int i = 1; i < m; ++i)
-        if (a * i % m == 1) return i;
-    return 1;
+    const float c1 = 0.923879533f, s1 = 0.382683432f, h = 0.707106781f;
+    const float c = e == 1 ? c1 : e == 2 ? h : e == 3 ? s1 : e == 6 ? -h : -c1;
+    float s = e == 1 ? s1 : e == 2 || e == 6 ? h : e == 3 ? c1 : -s1;
+    if (!INV) s = -s;  // forward W16^e = cos - i sin, inverse its conjugate
+    const auto x = !INV && e == 6 ? fmac_(a.y, -s, scale_(a.x, c)) : fmac_(a.x, c, scale_(a.y, -s));
+    return cmake<C>(x, e == 2 ? fmac_(a.x, s, scale_(a.y, c)) : fmac_(a.y, c, scale_(a.x, s)));
 }
-template <int A, int B>
-struct DftCoprime {
+template <>
+struct Dft<16> {
     template <bool INV, class C>
     static __device__ __forceinline__ void run(C* v)
     {
-        constexpr int E1 = B * inv_mod(B % A, A), E2 = A * inv_mod(A % B, B);
-        C t[A * B];
+        C y[16];
 #pragma unroll
-        for (int n1 = 0; n1 < A; ++n1) {
-            C u[B];
+        for (int n1 = 0; n1 < 4; ++n1) {
+            C t[4] = {v[n1], v[n1 + 4], v[n1 + 8], v[n1 + 12]};
+            Dft<4>::run<INV>(t);
 #pragma unroll
-            for (int n2 = 0; n2 < B; ++n2) u[n2] = v[(B * n1 + A * n2) % (A * B)];
-            Dft<B>::template run<INV>(u);
-#pragma unroll
-            for (int k2 = 0; k2 < B; ++k2) t[n1 * B + k2] = u[k2];
+            for (int k2 = 0; k2 < 4; ++k2)  // W16^4 = -+ i is taken in the second pass
+                y[n1 * 4 + k2] = n1 * k2 == 0 || n1 * k2 == 4 ? t[k2] : w16<INV>(t[k2], n1 * k2);
         }
 #pragma unroll
-        for (int k2 = 0; k2 < B; ++k2) {
+        for (int k2 = 0; k2 < 4; ++k2) {
+            C t[4] = {y[k2], y[4 + k2], y[8 + k2], y[12 + k2]};
+            Dft<4>::run<INV>(t, k2 == 2);
+#pragma unroll
+            for (int k1 = 0; k1 < 4; ++k1) v[k2 + 4 * k1] = t[k1];
+        }
+    }
+};
+
+// A stage of radix A, then radix B on its outputs.  Point r of v is index
+// j + r N / (A B); the second radix's butterflies take the same point o of B
+// first-radix butterflies, each times the twiddle inner(o, r2) applies.
+template <int A, int B, bool INV, class C, class In>
+__device__ __forceinline__ void dft_stage(C* v, In inner)
+{
+    if constexpr (B == 1) {
+        Dft<A>::template run<INV>(v);
+    } else {
+        C t[A * B];  // [o][r2]
+#pragma unroll
+        for (int r2 = 0; r2 < B; ++r2) {
             C u[A];
 #pragma unroll
-            for (int n1 = 0; n1 < A; ++n1) u[n1] = t[n1 * B + k2];
+            for (int r1 = 0; r1 < A; ++r1) u[r1] = v[r2 + B * r1];
             Dft<A>::template run<INV>(u);
 #pragma unroll
-            for (int k1 = 0; k1 < A; ++k1) v[(E1 * k1 + E2 * k2) % (A * B)] = u[k1];
+            for (int o = 0; o < A; ++o) t[o * B + r2] = r2 ? inner(u[o], o, r2) : u[o];
+        }
+#pragma unroll
+        for (int o = 0; o < A; ++o) {
+            Dft<B>::template run<INV>(t + o * B);
+#pragma unroll
+            for (int q = 0; q < B; ++q) v[o + A * q] = t[o * B + q];
         }
     }
-};
-template <>
-struct Dft<6> : DftCoprime<2, 3> {};
-template <>
-struct Dft<10> : DftCoprime<2, 5> {};
-template <>
-struct Dft<12> : DftCoprime<4, 3> {};
-template <>
-struct Dft<14> : DftCoprime<2, 7> {};
-template <>
-struct Dft<15> : DftCoprime<3, 5> {};
-
-// Radix A^2 (9, 16) in registers as A x A: DFT-A over n2 of v[n1 + A n2],
-// twiddle W^{n1 k2}, DFT-A over n1; output X[k2 + A k1].
-__device__ constexpr float sq_cos(int n, int e)
-{
-    if (n == 16) {
-        e %= 16;
-        const float c[16] = {1.f, 0.92387953251128674f, 0.70710678118654752f, 0.38268343236508977f,
-                             0.f, -0.38268343236508977f, -0.70710678118654752f, -0.92387953251128674f,
-                             -1.f, -0.92387953251128674f, -0.70710678118654752f, -0.38268343236508977f,
-                             0.f, 0.38268343236508977f, 0.70710678118654752f, 0.92387953251128674f};
-        return c[e];
-    }
-    const float c[9] = {1.f, 0.76604444311897804f, 0.17364817766693035f, -0.5f, -0.93969262078590838f,
-                        -0.93969262078590838f, -0.5f, 0.17364817766693035f, 0.76604444311897804f};
-    return c[e % 9];
 }
-__device__ constexpr float sq_sin(int n, int e)
-{
-    if (n == 16) return sq_cos(16, e + 12);  // sin(x) = cos(x - pi/2)
-    const float s[9] = {0.f, 0.64278760968653933f, 0.98480775301220806f, 0.86602540378443865f, 0.34202014332566873f,
-                        -0.34202014332566873f, -0.86602540378443865f, -0.98480775301220806f, -0.64278760968653933f};
-    return s[e % 9];
-}
-template <int A>
-struct DftSquare {
-    template <bool INV, class C>
-    static __device__ __forceinline__ void run(C* v)
-    {
-        C y[A * A];
-#pragma unroll
-        for (int n1 = 0; n1 < A; ++n1) {
-            C t[A];
-#pragma unroll
-            for (int n2 = 0; n2 < A; ++n2) t[n2] = v[n1 + A * n2];
-            Dft<A>::template run<INV>(t);
-#pragma unroll
-            for (int k2 = 0; k2 < A; ++k2) {
-                const int e = n1 * k2;
-                if (e == 0) y[n1 * A + k2] = t[k2];
-                else if (A == 4 && e == 4) y[n1 * A + k2] = t[k2];  // -+ i, taken in the second pass
-                else y[n1 * A + k2] = cmul_cs<INV>(t[k2], sq_cos(A * A, e), sq_sin(A * A, e));
-            }
-        }
-#pragma unroll
-        for (int k2 = 0; k2 < A; ++k2) {
-            C t[A];
-#pragma unroll
-            for (int n1 = 0; n1 < A; ++n1) t[n1] = y[n1 * A + k2];
-            if constexpr (A == 4) Dft<4>::template run<INV>(t, k2 == 2);
-            else Dft<A>::template run<INV>(t);
-#pragma unroll
-            for (int k1 = 0; k1 < A; ++k1) v[k2 + A * k1] = t[k1];
-        }
-    }
-};
-template <>
-struct Dft<9> : DftSquare<3> {};
-template <>
-struct Dft<16> : DftSquare<4> {};
 
 // ------------------------------------------------------------------- stages
 template <int V>
@@ -407,14 +369,15 @@ __device__ __forceinline__ int smem_at(int p, int i, int ps, int is, int padsh)
     return p * ps + i * is + (padsh ? (i >> padsh) * is : 0);
 }
 
-template <int R, bool PF, bool INV, class Load, class Store>
+template <int A, int B, bool PF, bool INV, class Load, class Store>
 __device__ __forceinline__ void fft_stage(int n, int P, int ps, int is, int padsh, int Ns, bool first, bool last,
                                           const float2* __restrict__ tw, const float2* src, float2* dst,
                                           Load& load, Store& store)
 {
+    constexpr int R = A * B;
     const int nr = n / R;
     const int total = P * nr;
-    const int twstride = n / (Ns * R);
+    const int tw1 = n / (Ns * A), tw2 = nr / Ns;  // twiddle strides of the two radices
     for (int t = threadIdx.x; t < total; t += blockDim.x) {
         int p, j;
         if (PF) { p = t % P; j = t / P; }
@@ -428,12 +391,9 @@ __device__ __forceinline__ void fft_stage(int n, int P, int ps, int is, int pads
         }
         if (jm) {
 #pragma unroll
-            for (int r = 1; r < R; ++r) {
-                const float2 w = tw[jm * r * twstride];
-                v[r] = INV ? cmulc(v[r], w) : cmul(v[r], w);
-            }
+            for (int r = B; r < R; ++r) v[r] = cmul_tw<INV>(v[r], tw[jm * (r / B) * tw1]);
         }
-        Dft<R>::template run<INV>(v);
+        dft_stage<A, B, INV>(v, [&](float2 u, int o, int r2) { return cmul_tw<INV>(u, tw[(jm + o * Ns) * r2 * tw2]); });
         const int base = (j - jm) * R + jm;
 #pragma unroll
         for (int r = 0; r < R; ++r) {
@@ -453,30 +413,31 @@ __device__ void fft_run(const FftPlan& pl, const float2* __restrict__ tw, float2
                         int P, int ps, int is, Load load, Store store, int padsh = 0)
 {
     int Ns = 1;
-    for (int s = 0; s < pl.nst; ++s) {
-        const bool first = (s == 0), last = (s == pl.nst - 1);
+    for (int s = 0; s < pl.q.nst; ++s) {
+        const bool first = (s == 0), last = (s == pl.q.nst - 1);
         const float2* src = first ? nullptr : (((s - 1) & 1) ? bufB : bufA);
         float2* dst = (s & 1) ? bufB : bufA;
-        auto stage = [&](auto RR) {
-            fft_stage<decltype(RR)::value, PF, INV>(pl.n, P, ps, is, padsh, Ns, first, last, tw, src, dst, load, store);
+        auto stage = [&](auto AA, auto BB) {
+            fft_stage<decltype(AA)::value, decltype(BB)::value, PF, INV>(pl.n, P, ps, is, padsh, Ns, first, last, tw,
+                                                                         src, dst, load, store);
         };
-        switch (pl.rad[s]) {
-            case 2: stage(IntC<2>{}); break;
-            case 3: stage(IntC<3>{}); break;
-            case 4: stage(IntC<4>{}); break;
-            case 5: stage(IntC<5>{}); break;
-            case 6: stage(IntC<6>{}); break;
-            case 7: stage(IntC<7>{}); break;
-            case 8: stage(IntC<8>{}); break;
-            case 9: stage(IntC<9>{}); break;
-            case 10: stage(IntC<10>{}); break;
-            case 12: stage(IntC<12>{}); break;
-            case 14: stage(IntC<14>{}); break;
-            case 15: stage(IntC<15>{}); break;
-            default: stage(IntC<16>{}); break;
+        switch (pl.q.a[s] * 16 + pl.q.b[s]) {
+            case 2 * 16 + 1: stage(IntC<2>{}, IntC<1>{}); break;
+            case 2 * 16 + 3: stage(IntC<2>{}, IntC<3>{}); break;
+            case 2 * 16 + 5: stage(IntC<2>{}, IntC<5>{}); break;
+            case 2 * 16 + 7: stage(IntC<2>{}, IntC<7>{}); break;
+            case 3 * 16 + 1: stage(IntC<3>{}, IntC<1>{}); break;
+            case 3 * 16 + 3: stage(IntC<3>{}, IntC<3>{}); break;
+            case 3 * 16 + 5: stage(IntC<3>{}, IntC<5>{}); break;
+            case 4 * 16 + 1: stage(IntC<4>{}, IntC<1>{}); break;
+            case 4 * 16 + 3: stage(IntC<4>{}, IntC<3>{}); break;
+            case 5 * 16 + 1: stage(IntC<5>{}, IntC<1>{}); break;
+            case 7 * 16 + 1: stage(IntC<7>{}, IntC<1>{}); break;
+            case 8 * 16 + 1: stage(IntC<8>{}, IntC<1>{}); break;
+            default: stage(IntC<16>{}, IntC<1>{}); break;
         }
         __syncthreads();
-        Ns *= pl.rad[s];
+        Ns *= pl.q.rad(s);
     }
 }
 
@@ -484,7 +445,7 @@ __device__ void fft_run(const FftPlan& pl, const float2* __restrict__ tw, float2
 // buffer of the pair (the one the last stage does not read).
 __device__ __forceinline__ float2* fft_out_buf(const FftPlan& pl, float2* bufA, float2* bufB)
 {
-    return ((pl.nst - 1) & 1) ? bufB : bufA;
+    return ((pl.q.nst - 1) & 1) ? bufB : bufA;
 }
 
 // Two real pencils a, b packed as z = a + i b and transformed together; this

@@ -15,26 +15,26 @@ __device__ __forceinline__ void prefetch_l2(const void* p, unsigned bytes)
 {
     asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(p), "r"(bytes) : "memory");
 }
-// --------------------------------------------------------------- k_sigma --
 // ------------------------------------------------------------------ k_st --
 // Compiled form of the stress update, one group of fields per block: NF = 9 the
-// normal stresses (G 0..8), NF = 6 a shear stress (xz, xy, yz; G 9..26).  A block owns four y rows and all z of one x; k_dz then takes the z
+// normal stresses (G 0..8), NF = 6 a shear stress (xz, xy, yz; G 9..26).  A block
+// owns four or eight y rows and all z of one x; k_dz then takes the z
 // derivatives.  (One block running the groups one after another and the z
 // derivatives at the end measured 2.2 ms at 256^3, 0.57 of them the z pass on a
 // third of its threads.)
 //
-// Rows 0 + 2 i and 1 + 3 i of a field are the two pencils of a packed pair
+// Rows 0 + i 1 and 2 + i 3 of a field are the two pencils of a packed pair
 // (fft_pair.cuh): one thread transforms all four rows, and the slot its
-// inverse leaves at height z holds rows 0, 1 in the first plane and 2, 3 in the
-// second, so the update runs on pairs of rows in packed arithmetic.  C2R by the Hermitian extension: a
-// butterfly's points below n/2 are loaded (two 16-byte loads of one sector: one 32-byte load per point
-// measured 0.72 against 0.57 ms for the normal stresses), those
-// above are the mirror of what the butterfly n/R - j loaded and come by
-// shuffle where the butterflies of a pencil are 8 or 16 neighbouring lanes (a
-// second load otherwise: 2.65 against 2.2 ms).  With eight rows (Q = 2) the two
-// row quads of a butterfly are neighbouring lanes and read 64 bytes of a line
-// between them: a warp's load touches 16 lines instead of 32 (shear 0.68
-// against 0.78 ms at 256^3, the whole update 1.40 against 1.52).
+// inverse leaves at height z holds rows 0, 2 in the first plane and 1, 3 in the
+// second, so the update runs on pairs of rows in packed arithmetic.  C2R by the
+// Hermitian extension: a butterfly's points below n/2 are loaded (two 16-byte
+// loads of one sector: one 32-byte load per point measured 0.72 against 0.57 ms
+// for the normal stresses), those above are the mirror of what the butterfly
+// n/R - j loaded and come by shuffle where the threads of a pencil are 8, 16 or
+// 32 neighbouring lanes (a second load otherwise: 2.65 against 2.2 ms).  With
+// eight rows (Q = 2) the two row quads of a butterfly are neighbouring lanes and
+// read 64 bytes of a line between them: a warp's load touches 16 lines instead
+// of 32 (shear 0.68 against 0.78 ms at 256^3, the whole update 1.40 against 1.52).
 constexpr int st_threads(int n, int nf, int q) { return warps_up(nf * q * pair_tasks(n)); }
 constexpr size_t st_smem(int n, int nf, int q) { return 16 * ((size_t)nf * q * pair_slots_q(n, q) + tw_rows_size(n)); }
 // Blocks per SM the registers are sized for (256 points, normal stresses: two
@@ -45,6 +45,15 @@ constexpr int st_blocks(int n, int nf, int q)
     int b = (nf == 9 ? (q == 1 ? 16 : 18) : 20) / warps;
     if (b < 1) b = 1;
     return b < m ? b : m < 1 ? 1 : m;
+}
+// Whether a compiled z length takes sxy's two terms one after the other (see
+// stress_pair): the 5-smooth lengths from 96, 64 and 512.
+constexpr bool st_halves(int n)
+{
+    if (n < 96) return n == 64;
+    for (int r : {2, 3, 5})
+        while (n % r == 0) n /= r;
+    return n == 1;
 }
 
 __device__ __forceinline__ f2 bc(float a) { return pack2(a, a); }
@@ -62,24 +71,45 @@ __device__ __forceinline__ void put2(float* p, int n, bool second, f2 v)
     if (second) p[n] = x.y;
 }
 
-// Constant-Q set of a modulus for two rows (see qset_f).
-__device__ __forceinline__ void qset2(f2 rho, f2 c, f2 g, float w0, float inv_w0, f2 o[5])
+// Constant-Q set of one modulus for two rows from its effective velocity
+// c = v cos(pi g/2) (cuviscoelas_3D.cu:195-205): eta1 = -rho c g w0, eta2 =
+// rho c^2, eta3 = rho c^3 g / w0, tau1 = rho c g pi, tau2 = rho c^2 g^2 pi / w0.
+// c is built in FP64 at setup; the products are rebuilt here in FP32.  The last
+// factor of each comes apart (o = m f), for sums that round the product only
+// once.
+struct QSet {
+    f2 m[5], f[5], o[5];
+};
+__device__ __forceinline__ void qset2(QSet& s, f2 rho, f2 c, f2 g, float w0, float inv_w0)
 {
     const float pi = 3.1415926f;
-    const f2 rc = rho * c, rcg = rc * g, u = rcg * c;
-    o[0] = rcg * bc(-w0);
-    o[1] = rc * c;
-    o[2] = u * c * bc(inv_w0);
-    o[3] = rcg * bc(pi);
-    o[4] = u * g * bc(pi * inv_w0);
+    const f2 rc = rho * c, rc2 = rc * c;
+    s.m[0] = neg_(rc) * g;          s.f[0] = bc(w0);
+    s.m[1] = rc;                    s.f[1] = c;
+    s.m[2] = rc2 * c * g;           s.f[2] = bc(inv_w0);
+    s.m[3] = rc * g;                s.f[3] = bc(pi);
+    s.m[4] = rc2 * g * g * bc(pi);  s.f[4] = bc(inv_w0);
+#pragma unroll
+    for (int j = 0; j < 5; ++j) s.o[j] = s.m[j] * s.f[j];
 }
-__device__ __forceinline__ f2 dot3(const f2* a, f2 x, f2 y, f2 z) { return fma_(a[2], z, fma_(a[1], y, a[0] * x)); }
-__device__ __forceinline__ f2 dot2(const f2* a, f2 x, f2 y) { return fma_(a[4], y, a[3] * x); }
+// a13 - 2 a55 of two sets, the product of a13 (but that of eta2, which eta3
+// shares) not rounded by itself
+__device__ __forceinline__ f2 less13(const QSet& a, const QSet& s5, int j)
+{
+    return j == 1 ? fma_(bc(-2.f), s5.o[j], a.o[j]) : fma_(a.m[j], a.f[j], s5.o[j] * bc(-2.f));
+}
+__device__ __forceinline__ f2 dot3(const f2* a, f2 x, f2 y, f2 z, int v = 0)
+{
+    return v ? fma_(a[2], z, fma_(a[1], y, a[0] * x)) : fma_(a[2], z, fma_(a[0], x, a[1] * y));
+}
+__device__ __forceinline__ f2 dot2(const f2* a, f2 x, f2 y, int v = 0)
+{
+    return v ? fma_(a[4], y, a[3] * x) : fma_(a[3], x, a[4] * y);
+}
 
 // One C-PML term of a row pair: the slab's memory variable and loss potential
 // (second row n further on), loaded, then advanced by the term d and its new
-// potential qn.  Rows outside the slab (on0, on1) keep zero; st1: the second
-// row is not the last plane.
+// potential qn.  Rows outside the slab (on0, on1) keep zero.
 struct Term {
     f2 po, qo;
 };
@@ -88,14 +118,14 @@ __device__ __forceinline__ void term_load(Term& t, const float* ph, const float*
     t.qo = pack2(on0 ? q[0] : 0.f, on1 ? q[n] : 0.f);
     t.po = pack2(on0 ? ph[0] : 0.f, on1 ? ph[n] : 0.f);
 }
-__device__ __forceinline__ f2 term_step(const Term& t, float* ph, float* q, int n, bool on0, bool on1, bool st1, f2 a,
-                                        f2 b, f2 d, f2 qn, f2 dt, f2 inv_dt)
+__device__ __forceinline__ f2 term_step(const Term& t, float* ph, float* q, int n, bool on0, bool on1, f2 a, f2 b, f2 d,
+                                        f2 qn, f2 dt, f2 inv_dt)
 {
     const f2 T = fma_(qn - t.qo, inv_dt, d);
-    const f2 r = fma_(dt, neg_(fma_(a, t.po, b * T)), t.po);
+    const f2 r = fma_(dt, fma_(neg_(a), t.po, neg_(b) * T), t.po);  // pml_step
     const float2 rv = unpack2(r), qv = unpack2(qn);
     if (on0) { q[0] = qv.x; ph[0] = rv.x; }
-    if (on1 && st1) { q[n] = qv.y; ph[n] = rv.y; }
+    if (on1) { q[n] = qv.y; ph[n] = rv.y; }
     return sel2(on0, on1, r);
 }
 
@@ -169,18 +199,20 @@ __device__ __forceinline__ void inject(const KP& k, int x, int y0, int yv)
 __device__ __forceinline__ float z_term(const KP& k, float* ph, int x, int y, int z, float a, float b, float d)
 {
     const int is = slab_z(k, x, y, z);
-    const float old = ph[is], nw = old + k.dt * (-a * old - b * d);
+    const float nw = pml_step(ph[is], k.dt, a, b, d);
     ph[is] = nw;
     return d + nw;
 }
 
-// Stress update of one group at height z of rows y, y + 1 (constant-Q
+// Stress update of one group at height z of rows y, y + D (constant-Q
 // dispersion and loss, C-PML; cu:800-1015), in packed arithmetic; sv(f): the
-// group's real field f at the two rows.  Not for the last x or z plane.  The
-// C-PML terms sit behind branches that are uniform but for the z slab's edges;
-// loads of a row pair that the compiler can all issue before the first store
-// are what keeps the update fed.
-template <class SV>
+// group's real field f at the two rows.  Not for the last x or z plane, nor y =
+// ny - 1.  The C-PML terms sit behind branches that are uniform but for the z
+// slab's edges; loads of a row pair that the compiler can all issue before the
+// first store are what keeps the update fed.
+// HALVES: sxy takes its y and its x term one after the other, each with its own
+// part of the loss (dt L = ls (Qxy - Qxy_old), Qxy the sum of the two parts).
+template <int D, bool HALVES, class SV>
 __device__ __forceinline__ void stress_pair(const KP& k, int n, int grp, int x, int y, int z, SV sv)
 {
     const int nx = k.nx, ny = k.ny, pml = k.pml;
@@ -188,41 +220,44 @@ __device__ __forceinline__ void stress_pair(const KP& k, int n, int grp, int x, 
     // inv_dt enters only the loss terms (the spectral time derivative of the
     // constant-Q loss operator): their sign and presence follow the medium
     // (k.loss_scale: 1 viscoelastic, 0 dispersion only, -1 Q-compensated)
-    const f2 dt = bc(k.dt), inv_dt = bc(k.loss_scale / k.dt);
+    const f2 dt = bc(k.dt), ls = bc(k.loss_scale), inv_dt = bc(k.loss_scale / k.dt);
     const bool sx = in_slab(x, nx, pml);
-    const bool in1 = y + 1 < ny - 1;  // the last plane of an axis is never updated
+    const bool in1 = y + D < ny - 1;  // the last plane of an axis is never updated
+    const int nd = in1 ? D * n : 0;   // to the second row; the first one again where there is none
     const int ip = cell(k, x, y, z);
-    const bool sy0 = in_slab(y, ny, pml), sy1 = in_slab(y + 1, ny, pml), sz = in_slab(z, n, pml);
+    const bool sy0 = in_slab(y, ny, pml), sy1 = in1 && in_slab(y + D, ny, pml), sz = in_slab(z, n, pml);
     const int isx = sx ? slab_x(k, x, y, z) : 0, isz = sz ? slab_z(k, x, y, z) : 0;
-    // row y + 1 of the y slab is n further on; a pair whose first row is
+    // row y + D of the y slab is D n further on; a pair whose first row is
     // outside starts at its second
-    const int isy = sy0 ? slab_y(k, x, y, z) : sy1 ? slab_y(k, x, y + 1, z) - n : 0;
+    const int isy = sy0 ? slab_y(k, x, y, z) : sy1 ? slab_y(k, x, y + D, z) - D * n : 0;
     const bool sy = sy0 || sy1;
+    const int nz2 = in1 ? 2 * D * pml : 0;
     // every load of the cell pair is issued before its first store: the arrays
     // cannot alias, but through the parameter struct the compiler cannot know
     Term tm[8];
-    auto xload = [&](int i, float* ph, float* q) { term_load(tm[i], ph + isx, q + isx, n, true, true); };
-    auto yload = [&](int i, float* ph, float* q) { term_load(tm[i], ph + isy, q + isy, n, sy0, sy1); };
-    auto zload = [&](int i, float* ph, float* q) { term_load(tm[i], ph + isz, q + isz, 2 * pml, true, true); };
+    auto xload = [&](int i, float* ph, float* q) { term_load(tm[i], ph + isx, q + isx, nd, true, true); };
+    auto yload = [&](int i, float* ph, float* q) { term_load(tm[i], ph + isy, q + isy, D * n, sy0, sy1); };
+    auto zload = [&](int i, float* ph, float* q) { term_load(tm[i], ph + isz, q + isz, nz2, true, true); };
     auto xterm = [&](int i, float* ph, float* q, f2 a, f2 b, f2 d, f2 qn) {
-        return term_step(tm[i], ph + isx, q + isx, n, true, true, in1, a, b, d, qn, dt, inv_dt);
+        return term_step(tm[i], ph + isx, q + isx, nd, true, in1, a, b, d, qn, dt, inv_dt);
     };
     auto yterm = [&](int i, float* ph, float* q, f2 a, f2 b, f2 d, f2 qn) {
-        return term_step(tm[i], ph + isy, q + isy, n, sy0, sy1, in1, a, b, d, qn, dt, inv_dt);
+        return term_step(tm[i], ph + isy, q + isy, D * n, sy0, sy1, a, b, d, qn, dt, inv_dt);
     };
     auto zterm = [&](int i, float* ph, float* q, f2 a, f2 b, f2 d, f2 qn) {
-        return term_step(tm[i], ph + isz, q + isz, 2 * pml, true, true, in1, a, b, d, qn, dt, inv_dt);
+        return term_step(tm[i], ph + isz, q + isz, nz2, true, in1, a, b, d, qn, dt, inv_dt);
     };
+    auto yrow = [&](const float* p) { return pack2(p[y], p[in1 ? y + D : y]); };
     if (grp == 0) {
-        f2 sxx = rows2(k.s[0] + ip, n), syy = rows2(k.s[1] + ip, n), szz = rows2(k.s[2] + ip, n);
-        const f2 qx = rows2(k.Q[0] + ip, n), qy = rows2(k.Q[1] + ip, n), qz = rows2(k.Q[2] + ip, n);
-        const f2 rho = rows2_ro(k.mrho + ip, n), gp = rows2_ro(k.mgp + ip, n), gs = rows2_ro(k.mgs + ip, n);
-        const f2 c33 = rows2_ro(k.mc33 + ip, n), cs = rows2_ro(k.mcs + ip, n);
+        f2 sxx = rows2(k.s[0] + ip, nd), syy = rows2(k.s[1] + ip, nd), szz = rows2(k.s[2] + ip, nd);
+        const f2 qx = rows2(k.Q[0] + ip, nd), qy = rows2(k.Q[1] + ip, nd), qz = rows2(k.Q[2] + ip, nd);
+        const f2 rho = rows2_ro(k.mrho + ip, nd), gp = rows2_ro(k.mgp + ip, nd), gs = rows2_ro(k.mgs + ip, nd);
+        const f2 c33 = rows2_ro(k.mc33 + ip, nd), cs = rows2_ro(k.mcs + ip, nd);
         f2 c11 = c33, c13 = c33;
         const bool aniso = k.mc11 != k.mc33;
         if (aniso) {
-            c11 = rows2_ro(k.mc11 + ip, n);
-            c13 = rows2_ro(k.mc13 + ip, n);
+            c11 = rows2_ro(k.mc11 + ip, nd);
+            c13 = rows2_ro(k.mc13 + ip, nd);
         }
         if (sx) {
 #pragma unroll
@@ -236,20 +271,28 @@ __device__ __forceinline__ void stress_pair(const KP& k, int n, int grp, int x, 
             zload(6, k.phn[6], k.qn[6]);
             zload(7, k.phn[7], k.qn[7]);
         }
-        f2 a11[5], a33[5], a13[5], a12[5], s5[5];
-        qset2(rho, c33, gp, w0, inv_w0, a33);
-        if (aniso) {
-            qset2(rho, c11, gp, w0, inv_w0, a11);
-            qset2(rho, c13, gp, w0, inv_w0, a13);
-        } else {  // isotropic: one modulus
+        f2 a11[5], a33[5], a13[5], a12[5];
+        {
+            QSet s5, q;
+            qset2(s5, rho, cs, gs, w0, inv_w0);
+            qset2(q, rho, c33, gp, w0, inv_w0);
 #pragma unroll
-            for (int j = 0; j < 5; ++j) a11[j] = a13[j] = a33[j];
-        }
-        qset2(rho, cs, gs, w0, inv_w0, s5);
+            for (int j = 0; j < 5; ++j) {
+                a33[j] = a11[j] = q.o[j];
+                a12[j] = fma_(bc(-2.f), s5.o[j], q.o[j]);
+                a13[j] = less13(q, s5, j);
+            }
+            if (aniso) {
+                qset2(q, rho, c11, gp, w0, inv_w0);
 #pragma unroll
-        for (int j = 0; j < 5; ++j) {
-            a12[j] = fma_(bc(-2.f), s5[j], a11[j]);
-            a13[j] = fma_(bc(-2.f), s5[j], a13[j]);
+                for (int j = 0; j < 5; ++j) {
+                    a11[j] = q.o[j];
+                    a12[j] = fma_(bc(-2.f), s5.o[j], q.o[j]);
+                }
+                qset2(q, rho, c13, gp, w0, inv_w0);
+#pragma unroll
+                for (int j = 0; j < 5; ++j) a13[j] = less13(q, s5, j);
+            }
         }
         f2 X = sv(0), Y = sv(1), Z = sv(2);
         const f2 d11x = dot3(a11, X, Y, Z), d12x = dot3(a12, X, Y, Z), d13x = dot3(a13, X, Y, Z);
@@ -258,7 +301,7 @@ __device__ __forceinline__ void stress_pair(const KP& k, int n, int grp, int x, 
         const f2 d12y = dot3(a12, X, Y, Z), d11y = dot3(a11, X, Y, Z), d13y = dot3(a13, X, Y, Z);
         const f2 q12y = dot2(a12, X, Y), q11y = dot2(a11, X, Y), q13y = dot2(a13, X, Y);
         X = sv(6); Y = sv(7); Z = sv(8);
-        const f2 d13z = dot3(a13, X, Y, Z), d33z = dot3(a33, X, Y, Z);
+        const f2 d13z = dot3(a13, X, Y, Z), d33z = dot3(a33, X, Y, Z, 1);
         const f2 q13z = dot2(a13, X, Y), q33z = dot2(a33, X, Y);
         // loss: sum_terms tau-coefficient x (S - S_prev)/dt = (Q - Q_prev)/dt
         const f2 Qxx = q11x + q12y + q13z, Qyy = q12x + q11y + q13z, Qzz = q13x + q13y + q33z;
@@ -272,7 +315,7 @@ __device__ __forceinline__ void stress_pair(const KP& k, int n, int grp, int x, 
             tzz = tzz + xterm(2, k.phn[2], k.qn[2], ax, bx, d13x, q13x);
         }
         if (sy) {
-            const f2 a = rows2(k.ay + y, 1), b = rows2(k.by + y, 1);
+            const f2 a = yrow(k.ay), b = yrow(k.by);
             txx = txx + yterm(3, k.phn[3], k.qn[3], a, b, d12y, q12y);
             tyy = tyy + yterm(4, k.phn[4], k.qn[4], a, b, d11y, q11y);
             tzz = tzz + yterm(5, k.phn[5], k.qn[5], a, b, d13y, q13y);
@@ -284,22 +327,22 @@ __device__ __forceinline__ void stress_pair(const KP& k, int n, int grp, int x, 
             tyy = tyy + p;
             tzz = tzz + zterm(7, k.phn[7], k.qn[7], a, b, d33z, q33z);
         }
-        put2(k.s[0] + ip, n, in1, fma_(dt, txx, sxx));
-        put2(k.s[1] + ip, n, in1, fma_(dt, tyy, syy));
-        put2(k.s[2] + ip, n, in1, fma_(dt, tzz, szz));
-        put2(k.Q[0] + ip, n, in1, Qxx);
-        put2(k.Q[1] + ip, n, in1, Qyy);
-        put2(k.Q[2] + ip, n, in1, Qzz);
+        put2(k.s[0] + ip, nd, in1, fma_(dt, txx, sxx));
+        put2(k.s[1] + ip, nd, in1, fma_(dt, tyy, syy));
+        put2(k.s[2] + ip, nd, in1, fma_(dt, tzz, szz));
+        put2(k.Q[0] + ip, nd, in1, Qxx);
+        put2(k.Q[1] + ip, nd, in1, Qyy);
+        put2(k.Q[2] + ip, nd, in1, Qzz);
     } else {
         // shear: xz, xy, yz (groups 1, 2, 3), each of two terms; A: dz vx, dy
         // vx, dz vy (z, y, z slab), B: dx vz, dx vy, dy vz (x, x, y slab)
         const int c = grp == 1 ? 4 : grp == 2 ? 3 : 5;
         float* __restrict__ sg = k.s[c] + ip;
         float* __restrict__ qg = k.Q[c] + ip;
-        const f2 s_old = rows2(sg, n), q_old = rows2(qg, n);
+        const f2 s_old = rows2(sg, nd), q_old = rows2(qg, nd);
         f2 mu[5];
 #pragma unroll
-        for (int j = 0; j < 5; ++j) mu[j] = rows2_ro(k.MU[j] + ip, n);
+        for (int j = 0; j < 5; ++j) mu[j] = rows2_ro(k.MU[j] + ip, nd);
         const int mA = 2 * (grp - 1), mB = mA + 1;
         const bool onA = grp == 2 ? sy : sz, onB = grp == 3 ? sy : sx;
         float *phA = k.phs[mA], *qsA = k.qs[mA], *phB = k.phs[mB], *qsB = k.qs[mB];
@@ -318,34 +361,42 @@ __device__ __forceinline__ void stress_pair(const KP& k, int n, int grp, int x, 
         const f2 dB = dot3(mu, X, Y, Z);
         const f2 qB = dot2(mu, X, Y);
         const f2 Qs = qA + qB;
-        f2 T = fma_(Qs - q_old, inv_dt, dA + dB);
+        f2 pA = bc(0.f), pB = bc(0.f);
         if (onA) {
-            if (grp == 2) T = T + yterm(0, phA, qsA, rows2(k.ayh + y, 1), rows2(k.byh + y, 1), dA, qA);
-            else T = T + zterm(0, phA, qsA, bc(k.azh[z]), bc(k.bzh[z]), dA, qA);
+            if (grp == 2) pA = yterm(0, phA, qsA, yrow(k.ayh), yrow(k.byh), dA, qA);
+            else pA = zterm(0, phA, qsA, bc(k.azh[z]), bc(k.bzh[z]), dA, qA);
         }
         if (onB) {
-            if (grp == 3) T = T + yterm(1, phB, qsB, rows2(k.ayh + y, 1), rows2(k.byh + y, 1), dB, qB);
-            else T = T + xterm(1, phB, qsB, bc(k.axh[x]), bc(k.bxh[x]), dB, qB);
+            if (grp == 3) pB = yterm(1, phB, qsB, yrow(k.ayh), yrow(k.byh), dB, qB);
+            else pB = xterm(1, phB, qsB, bc(k.axh[x]), bc(k.bxh[x]), dB, qB);
         }
-        put2(sg, n, in1, fma_(dt, T, s_old));
-        put2(qg, n, in1, Qs);
+        f2 S;
+        if (HALVES && grp == 2) {
+            S = fma_(ls, qA - q_old, fma_(dt, dA + pA, s_old));
+            S = fma_(ls, qB, fma_(dt, dB + pB, S));
+        } else {
+            S = fma_(dt, fma_(Qs - q_old, inv_dt, dA + pA + dB + pB), s_old);
+        }
+        put2(sg, nd, in1, S);
+        put2(qg, nd, in1, Qs);
     }
 }
 
 template <int N, int NF, int Q>
 __global__ void __launch_bounds__(st_threads(N, NF, Q), st_blocks(N, NF, Q)) k_st(KP k)
 {
-    using F = PairFFT<N, NF * Q, false, false, Q>;
-    constexpr int NT = st_threads(N, NF, Q), R0 = F::R0, RL = F::RL, NR0 = N / R0, ROWS = 4 * Q;
-    constexpr bool SHFL = R0 % 2 == 0 && (NR0 * Q == 8 || NR0 * Q == 16 || NR0 * Q == 32);
-    constexpr int RM = pair_rmax(N);
+    using F = PairFFT<N, NF * Q, false, Q>;
+    constexpr int NT = st_threads(N, NF, Q), R0 = F::R0, NR0 = N / R0, ROWS = 4 * Q, LANES = F::T * Q;
+    static_assert(NT <= 1024, "threads of a block");
+    constexpr bool SHFL = R0 % 2 == 0 && F::K0 == 1 && (LANES == 8 || LANES == 16 || LANES == 32);
     extern __shared__ float4 smem4[];
     f2* buf = reinterpret_cast<f2*>(smem4);
     float4* tw = smem4 + F::PLANE;
+    const TwRows<N> W{tw};
     const int t = threadIdx.x, nx = k.nx, ny = k.ny, x = blockIdx.y;
     // the three shear blocks of a tile are neighbours: they share MU in L2
     const int y0 = ROWS * (NF == 9 ? blockIdx.x : blockIdx.x / 3);
-    const int yv = min(ROWS, ny - y0);  // rows of the tile inside the grid (even)  // rows of the tile inside the grid: 4 or 2
+    const int yv = min(ROWS, ny - y0);  // rows of the tile inside the grid (even)
     constexpr float inv_nz = 1.0f / N;
     const int grp = NF == 9 ? 0 : blockIdx.x % 3 + 1;
     if (x == nx - 1) {  // the last plane of an axis is never updated
@@ -354,14 +405,14 @@ __global__ void __launch_bounds__(st_threads(N, NF, Q), st_blocks(N, NF, Q)) k_s
     }
 
     int p0, j0;
-    const bool act0 = F::template task<0>(t, p0, j0);
-    if (!act0) { p0 = NF * Q - Q + t % Q; j0 = t / Q % NR0; }
-    const int f0 = p0 / Q, q0 = 4 * (p0 % Q);  // field and first row of the pair 
+    const bool act = F::task(t, p0, j0);
+    if (!act) { p0 = NF * Q - Q + t % Q; j0 = 0; }
+    const int f0 = p0 / Q, q0 = 4 * (p0 % Q);  // field and first row of the pair
 
-    c2 v[RM];
-    // 1. C2R along z of the group's fields (whole warps: lanes past the
-    //    last butterfly follow along for the shuffles)
-    if ((t & ~31) < NF * Q * NR0) {
+    c2 v[F::RM];
+    // 1. C2R along z of the group's fields (whole warps: lanes without a
+    //    butterfly follow along for the shuffles)
+    if ((t & ~31) < NF * Q * F::T) {
         const int o = (NF == 9 ? 0 : 3 + 6 * grp) + f0;
         const bool gz = is_gz(o);
         const float2* src = gz ? k.H[o == 7 ? 2 : o == 10 ? 0 : 1]
@@ -381,7 +432,7 @@ __global__ void __launch_bounds__(st_threads(N, NF, Q), st_blocks(N, NF, Q)) k_s
             if (gz) {
                 const float2 m = cscale(M[kk], inv_nz);
 #pragma unroll
-                for (int q = 0; q < 4; ++q) a[q] = cmul(a[q], m);
+                for (int q = 0; q < 4; ++q) a[q] = st_halves(N) ? cmul_m(a[q], m) : cmul(a[q], m);
             }
             if (kk == 0 || 2 * kk == N) {
 #pragma unroll
@@ -389,12 +440,13 @@ __global__ void __launch_bounds__(st_threads(N, NF, Q), st_blocks(N, NF, Q)) k_s
             }
         };
         auto direct = [](const float2 a[4]) {
-            return c2{pack2(a[0].x - a[2].y, a[1].x - a[3].y), pack2(a[0].y + a[2].x, a[1].y + a[3].x)};
+            return c2{pack2(a[0].x - a[1].y, a[2].x - a[3].y), pack2(a[0].y + a[1].x, a[2].y + a[3].x)};
         };
         auto mirror = [](const float2 a[4]) {
-            return c2{pack2(a[0].x + a[2].y, a[1].x + a[3].y), pack2(a[2].x - a[0].y, a[3].x - a[1].y)};
+            return c2{pack2(a[0].x + a[1].y, a[2].x + a[3].y), pack2(a[1].x - a[0].y, a[3].x - a[2].y)};
         };
         if constexpr (SHFL) {
+            if (j0 >= NR0) j0 = 0;  // a pencil's lanes past its last butterfly
             c2 m[R0 / 2];
             float2 a[4];
 #pragma unroll
@@ -403,10 +455,10 @@ __global__ void __launch_bounds__(st_threads(N, NF, Q), st_blocks(N, NF, Q)) k_s
                 v[r] = direct(a);
                 m[r] = mirror(a);
             }
-            const int from = (NR0 - j0) * Q + p0 % Q;  // the butterfly that holds the mirror points (lane 0: itself)
+            const int from = (NR0 - j0) * Q + p0 % Q;  // the butterfly that holds the mirror points (j0 = 0: itself)
             auto swap1 = [&](f2 own, f2 send) {
                 const float2 s = unpack2(send), w = unpack2(own);
-                const float p = __shfl_sync(0xffffffffu, s.x, from, NR0 * Q), q = __shfl_sync(0xffffffffu, s.y, from, NR0 * Q);
+                const float p = __shfl_sync(0xffffffffu, s.x, from, LANES), q = __shfl_sync(0xffffffffu, s.y, from, LANES);
                 return j0 ? pack2(p, q) : pack2(w.x, w.y);
             };
             c2 ny2 = m[0];
@@ -420,39 +472,35 @@ __global__ void __launch_bounds__(st_threads(N, NF, Q), st_blocks(N, NF, Q)) k_s
                 v[r] = c2{swap1(own.x, m[R0 - 1 - r].x), swap1(own.y, m[R0 - 1 - r].y)};
             }
         } else {
+            F::template each<0>(j0, [&](int m, int j) {
 #pragma unroll
-            for (int r = 0; r < R0; ++r) {
-                const int i = j0 + r * NR0;
-                float2 a[4];
-                rows(i <= N / 2 ? i : N - i, a);
-                const c2 d = direct(a), m = mirror(a);
-                v[r] = i <= N / 2 ? d : m;
-            }
+                for (int r = 0; r < R0; ++r) {
+                    const int i = j + r * NR0;
+                    float2 a[4];
+                    rows(i <= N / 2 ? i : N - i, a);
+                    const c2 d = direct(a), c = mirror(a);
+                    v[m * R0 + r] = i <= N / 2 ? d : c;
+                }
+            });
         }
     }
     // behind the loads in flight (ahead of them its dozens of requests held up
     // the first warp: 1.40 against 1.38 ms at 256^3, 130 against 119 us at 96^3)
     if (t == 0) prefetch_group(k, N, grp, x, y0, yv);
     TwRows<N>::template fill<NT>(tw, k.tw_z);
-    F::template first<true>(buf, t, v);
-    F::template finish<true>(TwRows<N>{tw}, buf, t, v);
-    {
-        // the last stage's points go back to the slots they came from
-        constexpr int D = F::template dist<F::NST - 1>();
-        int pl, jl;
-        if (F::template task<F::NST - 1>(t, pl, jl)) {
-#pragma unroll
-            for (int r = 0; r < RL; ++r) F::st(buf + F::slot(pl, jl) + r * D, v[r]);
-        }
-    }
+    if (F::SYNC0) __syncthreads();
+    F::template first<true>(W, buf, t, v);
+    F::template finish<true>(W, buf, t, v);
+    F::keep(buf, t, v);
     __syncthreads();
 
-    // 2. stress update of the group: a thread takes rows 2h, 2h + 1 at z
+    // 2. stress update of the group: a thread takes rows 0, 2 or 1, 3 of a
+    //    quad at z
     for (int w = t; w < ROWS / 2 * N; w += NT) {
-        const int h = (unsigned)w / N, z = w - h * N, y = y0 + 2 * h;
-        if (2 * h >= yv || z == N - 1) continue;
+        const int h = (unsigned)w / N, z = w - h * N, row = h / 2 * 4 + h % 2, y = y0 + row;
+        if (row >= yv || y == ny - 1 || z == N - 1) continue;
         const f2* S = buf + (h & 1) * F::PLANE + F::slot(h / 2, z);
-        stress_pair(k, N, grp, x, y, z, [&](int f) { return S[f * Q * F::SL]; });
+        stress_pair<2, st_halves(N)>(k, N, grp, x, y, z, [&](int f) { return S[f * Q * F::SL]; });
     }
     if constexpr (NF == 9) {
         __syncthreads();
@@ -471,7 +519,7 @@ constexpr size_t dz_smem(int n) { return 16 * ((size_t)kDzPairs * pair_slots(n) 
 constexpr int dz_blocks(int n)
 {
     const int warps = dz_threads(n) / 32;
-    int b = 65536 / ((pair_rmax(n) >= 10 ? 128 : 96) * dz_threads(n));
+    int b = 65536 / (128 * dz_threads(n));
     while (b > 1 && b * warps % 4) --b;
     return b < 1 ? 1 : b;
 }
@@ -479,60 +527,69 @@ constexpr int dz_blocks(int n)
 template <int N>
 __global__ void __launch_bounds__(dz_threads(N), dz_blocks(N)) k_dz(KP k)
 {
-    using D = PairFFT<N, kDzPairs, false, false>;
-    using I = PairFFT<N, kDzPairs, false, true>;
-    constexpr int NT = dz_threads(N), RM = pair_rmax(N), R0 = D::R0, RL = D::RL, NR0 = N / R0;
+    using D = PairFFT<N, kDzPairs, false>;
+    constexpr int NT = dz_threads(N), R0 = D::R0, RL = D::RL;
     extern __shared__ float4 smem4[];
     f2* buf = reinterpret_cast<f2*>(smem4);
-    float4* tw = smem4 + kDzPairs * pair_slots(N);
+    float4* tw = smem4 + D::PLANE;
+    const TwRows<N> W{tw};
     const int t = threadIdx.x, ny = k.ny, x = blockIdx.y, f = blockIdx.z;
     const float inv_n = 1.0f / N;
-    c2 v[RM];
+    c2 v[D::RM];
     int q, j;
-    if (D::template task<0>(t, q, j)) {
-        const int y0 = (blockIdx.x * kDzPairs + q) * 4, yv = ny - y0;
-        const float* p = k.s[f == 0 ? 2 : f == 1 ? 4 : 5] + cell(k, x, y0, j);
+    const bool act = D::task(t, q, j);
+    const int y0 = (blockIdx.x * kDzPairs + q) * 4, yv = ny - y0;
+    if (act) {
+        const float* s = k.s[f == 0 ? 2 : f == 1 ? 4 : 5] + cell(k, x, y0, 0);
+        D::template each<0>(j, [&](int m, int i) {
 #pragma unroll
-        for (int r = 0; r < R0; ++r) {
-            const int i = r * NR0;
-            v[r] = c2{yv > 0 ? pack2(p[i], p[i + N]) : bc(0.f), yv > 2 ? pack2(p[i + 2 * N], p[i + 3 * N]) : bc(0.f)};
-        }
+            for (int r = 0; r < R0; ++r) {
+                const float* p = s + i + r * (N / R0);
+                const bool r01 = yv > 0, r23 = yv > 2;
+                v[m * R0 + r] = c2{pack2(r01 ? p[0] : 0.f, r23 ? p[2 * N] : 0.f), pack2(r01 ? p[N] : 0.f, r23 ? p[3 * N] : 0.f)};
+            }
+        });
     }
     TwRows<N>::template fill<NT>(tw, k.tw_z);
-    D::template first<false>(buf, t, v);
-    D::template finish<false>(TwRows<N>{tw}, buf, t, v);
-    if (D::template task<D::NST - 1>(t, q, j)) {
+    if (D::SYNC0) __syncthreads();
+    D::template first<false>(W, buf, t, v);
+    D::template finish<false>(W, buf, t, v);
+    D::turn(buf, t, v);
+    if (act) {
         const float2* T = f == 0 ? k.Bz : k.Fz;
+        D::template each<0>(j, [&](int m, int i) {
 #pragma unroll
-        for (int r = 0; r < RL; ++r) {
-            const float2 m = cscale(__ldg(T + j + r * (N / RL)), inv_n);
-            v[r] = cmul_tw<false>(v[r], bc(m.x), bc(m.y));
-        }
+            for (int r = 0; r < R0; ++r) {
+                const float2 c = cscale(__ldg(T + i + r * (N / R0)), inv_n);
+                v[m * R0 + r] = cmul_m(v[m * R0 + r], bc(c.x), bc(c.y));
+            }
+        });
     }
     __syncthreads();
-    I::template first<true>(buf, t, v);
-    I::template finish<true>(TwGlobal<N>{k.tw_z}, buf, t, v);
-    if (I::template task<I::NST - 1>(t, q, j)) {
-        const int y0 = (blockIdx.x * kDzPairs + q) * 4, yv = ny - y0;
+    D::template first<true>(W, buf, t, v);
+    D::template finish<true>(W, buf, t, v);
+    if (act) {
         float* __restrict__ R = k.R[f == 0 ? 2 : f == 1 ? 0 : 1] + cell(k, x, y0, 0);
         float* __restrict__ ph = k.php[f == 0 ? 8 : f == 1 ? 2 : 5];  // pzz_z, pxz_z, pyz_z
         const float* pa = f == 0 ? k.azh : k.az;
         const float* pb = f == 0 ? k.bzh : k.bz;
+        D::template each<D::LAST>(j, [&](int m, int i0) {
 #pragma unroll
-        for (int r = 0; r < R0; ++r) {
-            const int i = j + r * NR0;
-            const float2 u = unpack2(v[r].x), w = unpack2(v[r].y);
-            float d[4] = {u.x, u.y, w.x, w.y};
-            if (x < k.nx - 1 && i < N - 1 && in_slab(i, N, k.pml)) {
-                const float a = pa[i], b = pb[i];
+            for (int r = 0; r < RL; ++r) {
+                const int i = i0 + r * (N / RL);
+                const float2 u = unpack2(v[m * RL + r].x), w = unpack2(v[m * RL + r].y);
+                float d[4] = {u.x, w.x, u.y, w.y};
+                if (x < k.nx - 1 && i < N - 1 && in_slab(i, N, k.pml)) {
+                    const float a = pa[i], b = pb[i];
+#pragma unroll
+                    for (int c = 0; c < 4; ++c)
+                        if (c < yv - 1) d[c] = z_term(k, ph, x, y0 + c, i, a, b, d[c]);
+                }
 #pragma unroll
                 for (int c = 0; c < 4; ++c)
-                    if (c < yv - 1) d[c] = z_term(k, ph, x, y0 + c, i, a, b, d[c]);
+                    if (c < yv) R[i + c * N] = d[c];
             }
-#pragma unroll
-            for (int c = 0; c < 4; ++c)
-                if (c < yv) R[i + c * N] = d[c];
-        }
+        });
     }
 }
 
@@ -550,7 +607,7 @@ __global__ void __launch_bounds__(kThreads, 2) k_sigma(KP k, int P)
     float2* tw = sm;
     float2* A = tw + n;
     float2* B = A + bufA;  // only with more than two stages
-    float* S = reinterpret_cast<float*>(B + (k.pz.nst > 2 ? bufA : 0));  // [9][P][np1]: the group's real fields
+    float* S = reinterpret_cast<float*>(B + (k.pz.q.nst > 2 ? bufA : 0));  // [9][P][np1]: the group's real fields
     const int x = blockIdx.y, y0 = blockIdx.x * P, yv = min(P, ny - y0), grp = blockIdx.z;
     if (x == nx - 1) {  // the last plane of an axis is never updated
         if (grp == 0 && threadIdx.x == 0) inject(k, x, y0, yv);
@@ -587,7 +644,7 @@ __global__ void __launch_bounds__(kThreads, 2) k_sigma(KP k, int P)
     for (int w = threadIdx.x; w < Qp * n; w += blockDim.x) {
         const int h = w / n, z = w - h * n;
         if (2 * h >= yv || z == n - 1) continue;
-        stress_pair(k, n, grp, x, y0 + 2 * h, z, [&](int f) {
+        stress_pair<1, false>(k, n, grp, x, y0 + 2 * h, z, [&](int f) {
             const float* p = S + (f * P + 2 * h) * np1 + z;
             return pack2(p[0], p[np1]);
         });
@@ -625,7 +682,7 @@ __global__ void __launch_bounds__(kThreads) k_dzr(KP k, int P)
     float* __restrict__ ph = k.php[f == 0 ? 8 : f == 1 ? 2 : 5];  // pzz_z, pxz_z, pyz_z
     const float* pa = f == 0 ? k.azh : k.az;
     const float* pb = f == 0 ? k.bzh : k.bz;
-    auto load_i = [&](int q, int i) -> float2 { return cmul(Zf[q * ps + i], cscale(T[i], inv_n)); };
+    auto load_i = [&](int q, int i) -> float2 { return cmul_m(Zf[q * ps + i], cscale(T[i], inv_n)); };
     auto store_i = [&](int q, int i, float2 v) {
         if (2 * q >= yv) return;
         const int y = y0 + 2 * q;
@@ -697,7 +754,7 @@ size_t smem_sigma(const KP& k, int P, bool rt)
 {
     if (!rt) return std::max(st_smem(k.nz, 9, P / 4), dz_smem(k.nz));
     const size_t bufA = (size_t)9 * (P / 2) * (k.nz + k.nz / 16);
-    const int nb = k.pz.nst > 2 ? 2 : 1;
+    const int nb = k.pz.q.nst > 2 ? 2 : 1;
     return sizeof(float2) * (k.nz + nb * bufA) + sizeof(float) * (size_t)9 * P * (k.nz + 1);
 }
 

@@ -58,18 +58,17 @@ __global__ void __launch_bounds__(kThreads) k_fz(KP k, int P)
 #endif  // QVTI_PART == 0
 
 // ------------------------------------------------------------------ k_fp --
-// Compiled form of k_fz: 16 rows as four packed pairs, rows 0 + 2 i and 1 + 3 i
+// Compiled form of k_fz: 16 rows as four packed pairs, rows 0 + i 1 and 2 + i 3
 // of a quad in each (fft_pair.cuh), the four quads of a butterfly on
 // neighbouring lanes; the unpacking reads the planes pair-fastest, so four
-// lanes write one 128-byte line of the spectrum (96 against 118 us for k_fz at
-// 256^3, 27 against 40 at 150^3, 359 against 439 at 512x512x256).
+// lanes write one 128-byte line of the spectrum.
 constexpr int kFpPairs = 4;
 constexpr int fp_threads(int n) { return warps_up(kFpPairs * pair_tasks(n)); }
 constexpr size_t fp_smem(int n) { return 16 * ((size_t)kFpPairs * pair_slots_q(n, kFpPairs) + tw_rows_size(n)); }
 constexpr int fp_blocks(int n)
 {
     const int warps = fp_threads(n) / 32;
-    int b = 65536 / ((pair_rmax(n) >= 10 ? 128 : 80) * fp_threads(n));
+    int b = 65536 / (128 * fp_threads(n));
     while (b > 1 && b * warps % 4) --b;
     return b < 1 ? 1 : b;
 }
@@ -77,31 +76,31 @@ constexpr int fp_blocks(int n)
 template <int N>
 __global__ void __launch_bounds__(fp_threads(N), fp_blocks(N)) k_fp(KP k)
 {
-    using F = PairFFT<N, kFpPairs, false, false, kFpPairs>;
-    constexpr int NT = fp_threads(N), RM = pair_rmax(N), R0 = F::R0, RL = F::RL;
+    using F = PairFFT<N, kFpPairs, false, kFpPairs>;
+    constexpr int NT = fp_threads(N), R0 = F::R0;
     extern __shared__ float4 smem4[];
     f2* buf = reinterpret_cast<f2*>(smem4);
     float4* tw = smem4 + F::PLANE;
     const int t = threadIdx.x, x = blockIdx.y, y0 = blockIdx.x * 4 * kFpPairs;
-    c2 v[RM];
+    c2 v[F::RM];
     int p, j;
-    if (F::template task<0>(t, p, j)) {
+    if (F::task(t, p, j)) {
         const int left = k.ny - y0 - 4 * p;  // rows of the quad inside the grid: 4 or more, 2, none
-        const float* s = k.v[blockIdx.z] + cell(k, x, y0 + 4 * p, j);
+        const float* s = k.v[blockIdx.z] + cell(k, x, y0 + 4 * p, 0);
+        F::template each<0>(j, [&](int m, int i) {
 #pragma unroll
-        for (int r = 0; r < R0; ++r) {
-            const float* a = s + r * (N / R0);
-            v[r] = c2{left > 0 ? pack2(a[0], a[N]) : pack2(0.f, 0.f), left > 2 ? pack2(a[2 * N], a[3 * N]) : pack2(0.f, 0.f)};
-        }
+            for (int r = 0; r < R0; ++r) {
+                const float* a = s + i + r * (N / R0);
+                const bool r01 = left > 0, r23 = left > 2;
+                v[m * R0 + r] = c2{pack2(r01 ? a[0] : 0.f, r23 ? a[2 * N] : 0.f), pack2(r01 ? a[N] : 0.f, r23 ? a[3 * N] : 0.f)};
+            }
+        });
     }
     TwRows<N>::template fill<NT>(tw, k.tw_z);
-    F::template first<false>(buf, t, v);
+    if (F::SYNC0) __syncthreads();
+    F::template first<false>(TwRows<N>{tw}, buf, t, v);
     F::template finish<false>(TwRows<N>{tw}, buf, t, v);
-    constexpr int D = F::template dist<F::NST - 1>();
-    if (F::template task<F::NST - 1>(t, p, j)) {
-#pragma unroll
-        for (int r = 0; r < RL; ++r) F::st(buf + F::slot(p, j) + r * D, v[r]);
-    }
+    F::keep(buf, t, v);
     __syncthreads();
     float2* H = k.H[blockIdx.z];
     const f2 half = pack2(0.5f, 0.5f);
@@ -109,12 +108,12 @@ __global__ void __launch_bounds__(fp_threads(N), fp_blocks(N)) k_fp(KP k)
         const int q = w % kFpPairs, kz = (unsigned)w / kFpPairs, y = y0 + 4 * q;
         if (y >= k.ny) continue;
         const c2 z = F::ld(buf + F::slot(q, kz)), m = F::ld(buf + F::slot(q, kz ? N - kz : 0));
-        // rows 0, 1: (Z + conj Z(-k)) / 2; rows 2, 3: (Z - conj Z(-k)) / 2i
+        // rows 0, 2: (Z + conj Z(-k)) / 2; rows 1, 3: (Z - conj Z(-k)) / 2i
         const float2 ar = unpack2((z.x + m.x) * half), ai = unpack2((z.y - m.y) * half);
         const float2 br = unpack2((z.y + m.y) * half), bi = unpack2((m.x - z.x) * half);
         float4* to = reinterpret_cast<float4*>(H + spec(k, kz, x, y));
-        to[0] = make_float4(ar.x, ai.x, ar.y, ai.y);
-        if (y + 2 < k.ny) to[1] = make_float4(br.x, bi.x, br.y, bi.y);
+        to[0] = make_float4(ar.x, ai.x, br.x, bi.x);
+        if (y + 2 < k.ny) to[1] = make_float4(ar.y, ai.y, br.y, bi.y);
     }
 }
 
@@ -165,7 +164,7 @@ __global__ void __launch_bounds__(kCyThreads) k_cy(KP k, int L, long long line0,
             const float2* T = c == 1 ? k.Fy : k.By;
             const float inv_n = 1.0f / ((float)n * (float)k.nz);
             float2* yd = k.Yv[c] + off;
-            auto load_d = [&](int p, int i) -> float2 { return cmul(C[p * n + i], cscale(T[i], inv_n)); };
+            auto load_d = [&](int p, int i) -> float2 { return cmul_m(C[p * n + i], cscale(T[i], inv_n)); };
             auto store_d = [&](int p, int i, float2 v) {
                 if (p < lv) yd[(long long)p * n + i] = v;
             };
@@ -179,17 +178,14 @@ __global__ void __launch_bounds__(kCyThreads) k_cy(KP k, int L, long long line0,
 // ------------------------------------------------------------------ k_cp --
 // Compiled form of k_cy: eight lines as four packed pairs (fft_pair.cuh), the
 // y derivative of the forward pass taken from the registers the transform
-// ends in (reversed radices), as in k_dv.
+// ends in.
 constexpr int kCpPairs = 4;
 constexpr int cp_threads(int n) { return warps_up(kCpPairs * pair_tasks(n)); }
 constexpr size_t cp_smem(int n) { return 16 * ((size_t)kCpPairs * pair_slots(n) + tw_rows_size(n)); }
-// (0.56 ms for the inverse pass at 256^3, 5.1 TB/s, where the scalar kernel took
-// 0.54; 1.98 against 3.57 ms at 512x512x256, 48 against 77 us at 96x150x96, and
-// the forward pass 0.10 against 0.135 ms at 256^3.)
 constexpr int cp_blocks(int n)
 {
     const int warps = cp_threads(n) / 32;
-    int b = 65536 / ((pair_rmax(n) >= 14 ? 128 : pair_rmax(n) >= 10 ? 96 : 80) * cp_threads(n));
+    int b = 65536 / (128 * cp_threads(n));
     while (b > 1 && b * warps % 4) --b;
     return b < 1 ? 1 : b;
 }
@@ -197,62 +193,66 @@ constexpr int cp_blocks(int n)
 template <int N, bool INV>
 __global__ void __launch_bounds__(cp_threads(N), cp_blocks(N)) k_cp(KP k, long long line0, long long line_end)
 {
-    using F = PairFFT<N, kCpPairs, false, false>;
-    constexpr int NT = cp_threads(N), RM = pair_rmax(N), R0 = F::R0, RL = F::RL;
+    using F = PairFFT<N, kCpPairs, false>;
+    constexpr int NT = cp_threads(N), R0 = F::R0, RL = F::RL;
     extern __shared__ float4 smem4[];
     f2* buf = reinterpret_cast<f2*>(smem4);
-    float4* tw = smem4 + kCpPairs * pair_slots(N);
+    float4* tw = smem4 + F::PLANE;
+    const TwRows<N> W{tw};
     const int c = blockIdx.y, t = threadIdx.x;
     const long long first = line0 + (long long)blockIdx.x * 2 * kCpPairs, left = line_end - first;
     const float2* src = (INV ? k.G[c_gxy[c]] : k.H[c]) + first * N;
     float2* dst = (INV ? k.G[c_gxy[c]] : k.Hy[c]) + first * N;
-    c2 v[RM];
+    c2 v[F::RM];
     int p, j;
-    if (F::template task<0>(t, p, j)) {
-        const float2* a = src + 2 * p * N + j;
-        const bool in0 = 2 * p < left, in1 = 2 * p + 1 < left;
+    const bool act = F::task(t, p, j);
+    const bool in0 = 2 * p < left, in1 = 2 * p + 1 < left;
+    if (act)
+        F::template each<0>(j, [&](int m, int i) {
+            const float2* a = src + 2 * p * N + i;
 #pragma unroll
-        for (int r = 0; r < R0; ++r) {
-            const float2 x = in0 ? a[r * (N / R0)] : make_float2(0.f, 0.f);
-            const float2 y = in1 ? a[r * (N / R0) + N] : make_float2(0.f, 0.f);
-            v[r] = c2{pack2(x.x, y.x), pack2(x.y, y.y)};
-        }
-    }
+            for (int r = 0; r < R0; ++r) {
+                const float2 x = in0 ? a[r * (N / R0)] : make_float2(0.f, 0.f);
+                const float2 y = in1 ? a[r * (N / R0) + N] : make_float2(0.f, 0.f);
+                v[m * R0 + r] = c2{pack2(x.x, y.x), pack2(x.y, y.y)};
+            }
+        });
     TwRows<N>::template fill<NT>(tw, k.tw_y);
-    F::template first<INV>(buf, t, v);
-    F::template finish<INV>(TwRows<N>{tw}, buf, t, v);
-    auto store = [&](float2* to, int pp, int i, c2 w) {
-        const float2 re = unpack2(w.x), im = unpack2(w.y);
-        if (2 * pp < left) to[2 * pp * N + i] = make_float2(re.x, im.x);
-        if (2 * pp + 1 < left) to[(2 * pp + 1) * N + i] = make_float2(re.y, im.y);
-    };
-    const bool actl = F::template task<F::NST - 1>(t, p, j);
-    if (actl) {
+    if (F::SYNC0) __syncthreads();
+    F::template first<INV>(W, buf, t, v);
+    F::template finish<INV>(W, buf, t, v);
+    auto store = [&](float2* to) {
+        if (act)
+            F::template each<F::LAST>(j, [&](int m, int i) {
 #pragma unroll
-        for (int r = 0; r < RL; ++r) store(dst, p, j + r * (N / RL), v[r]);
-    }
+                for (int r = 0; r < RL; ++r) {
+                    const float2 re = unpack2(v[m * RL + r].x), im = unpack2(v[m * RL + r].y);
+                    const int at = 2 * p * N + i + r * (N / RL);
+                    if (in0) to[at] = make_float2(re.x, im.x);
+                    if (in1) to[at + N] = make_float2(re.y, im.y);
+                }
+            });
+    };
+    store(dst);
     if constexpr (!INV) {
         // the y derivative with the identity dispersion operator, scaled by
         // 1/(ny nz) like a field of the x and y passes (1/ntp times the x round
         // trip's nx): dy vy (c = 1, forward shift), dy vx and dy vz (backward)
-        using I = PairFFT<N, kCpPairs, false, true>;
         const float2* T = c == 1 ? k.Fy : k.By;
         const float inv_n = 1.0f / ((float)N * (float)k.nz);
-        if (actl) {
+        F::turn(buf, t, v);
+        if (act)
+            F::template each<0>(j, [&](int m, int i) {
 #pragma unroll
-            for (int r = 0; r < RL; ++r) {
-                const float2 m = cscale(__ldg(T + j + r * (N / RL)), inv_n);
-                v[r] = cmul_tw<false>(v[r], pack2(m.x, m.x), pack2(m.y, m.y));
-            }
-        }
+                for (int r = 0; r < R0; ++r) {
+                    const float2 f = cscale(__ldg(T + i + r * (N / R0)), inv_n);
+                    v[m * R0 + r] = cmul_m(v[m * R0 + r], pack2(f.x, f.x), pack2(f.y, f.y));
+                }
+            });
         __syncthreads();
-        I::template first<true>(buf, t, v);
-        I::template finish<true>(TwGlobal<N>{k.tw_y}, buf, t, v);
-        if (I::template task<I::NST - 1>(t, p, j)) {
-            float2* yd = k.Yv[c] + first * N;
-#pragma unroll
-            for (int r = 0; r < R0; ++r) store(yd, p, j + r * (N / R0), v[r]);
-        }
+        F::template first<true>(W, buf, t, v);
+        F::template finish<true>(W, buf, t, v);
+        store(k.Yv[c] + first * N);
     }
 }
 
@@ -271,7 +271,7 @@ __global__ void __launch_bounds__(kThreads) k_mx(KP k, int P, int kz0)
     // the second transform buffer exists only for transforms of more than
     // two stages (a two-stage transform reads its input through `load` and
     // writes its output through `store`)
-    const int nbuf = k.px.nst > 2 ? 2 : 1;
+    const int nbuf = k.px.q.nst > 2 ? 2 : 1;
     float2* tw = sm;
     float2* tFx = tw + n;
     float2* tBx = tFx + n;
@@ -339,21 +339,17 @@ __global__ void __launch_bounds__(kThreads) k_mx(KP k, int P, int kz0)
 
 // ------------------------------------------------------------------ k_mp --
 // Compiled form of k_mx: the same job on pairs of y rows in packed arithmetic
-// (fft_pair.cuh).  The forward transform's last stage leaves V at exactly the
-// points each inverse's first stage takes, so V stays in registers for all
-// seven fields and only the exchanges of the transforms go through shared
-// memory (k_mx, with V there too, took 0.50 ms at 256^3 against 0.42, 47 against 29
-// us at 96^3, 3.5 against 2.46 ms at 512x512x256).
-// 16 y (128-byte rows); 8 where three stages make a block of many small
-// butterflies (512x512x256: 2.23 against 2.46 ms, 384x384x256 1.48 against 1.59).
+// (fft_pair.cuh).  V is turned once into the points each inverse's first stage
+// takes, so it stays in registers for all seven fields and only the exchanges
+// of the transforms go through shared memory.
+// 16 y (128-byte rows); 8 at three stages.
 constexpr int mp_pairs(int n) { return mp_rows(n) / 2; }
 constexpr int mp_threads(int n) { return warps_up(mp_pairs(n) * pair_tasks(n)); }
 constexpr size_t mp_smem(int n) { return 16 * ((size_t)mp_pairs(n) * pair_slots(n) + 2 * (size_t)n) + 4 * (size_t)n; }
-// V and the working butterfly: 8 registers a point (radix 16: 168 registers and
-// three blocks measured 0.418 ms at 256^3, 128 and spills 0.447).
+// V and the working butterflies: 8 registers a point.
 constexpr int mp_blocks(int n)
 {
-    const int regs = pair_rmax(n) >= 14 ? 168 : pair_rmax(n) >= 10 ? 128 : 96;
+    const int regs = pair_rmax(n) >= 14 ? 168 : 128;
     const int b = 65536 / (regs * mp_threads(n)), m = (int)(220 * 1024 / (mp_smem(n) + 1024));
     return b < 1 ? 1 : b < m ? b : m;
 }
@@ -361,56 +357,53 @@ constexpr int mp_blocks(int n)
 template <int N>
 __global__ void __launch_bounds__(mp_threads(N), mp_blocks(N)) k_mp(KP k, int kz0)
 {
-    constexpr int PP = mp_pairs(N), NT = mp_threads(N), RM = pair_rmax(N);
-    using F = PairFFT<N, PP, true, false>;
-    using I = PairFFT<N, PP, true, true>;
+    constexpr int PP = mp_pairs(N), NT = mp_threads(N);
+    using F = PairFFT<N, PP, true>;
     constexpr int R0 = F::R0, RL = F::RL;
     extern __shared__ float4 smem4[];
     f2* buf = reinterpret_cast<f2*>(smem4);
     float4* tw = smem4 + PP * pair_slots(N);
-    float4* tx = tw + N;                                 // the component's x shift / ntp, doubled like the twiddles
-    float* tk = reinterpret_cast<float*>(tx + N);        // kx^2
+    float4* tx = tw + N;                                 // the component's x shift, doubled like the twiddles
+    float* tk = reinterpret_cast<float*>(tx + N);        // |kx|
+    const TwAll<N> W{tw};
     const int kz = kz0 + blockIdx.y, y0 = blockIdx.x * 2 * PP, c = blockIdx.z % 3, t = threadIdx.x;
     const int part = blockIdx.z / 3, parts = gridDim.z / 3;  // of the three directions of c
     const float sc = k.inv_ntp;
-    c2 v[RM], V[RM];
+    c2 v[F::RM], V[F::RM];
     int p, j;
-    const bool act0 = F::template task<0>(t, p, j);
-    if (act0) {
-        const int y = y0 + 2 * p;
-        const float4* src = reinterpret_cast<const float4*>(k.Hy[c] + spec(k, kz, j, y));
-        const bool in = y < k.ny;
+    const bool act = F::task(t, p, j);
+    const int y = y0 + 2 * p;
+    const bool in = y < k.ny;
+    if (act)
+        F::template each<0>(j, [&](int m, int i) {
+            const float4* src = reinterpret_cast<const float4*>(k.Hy[c] + spec(k, kz, i, y));
 #pragma unroll
-        for (int r = 0; r < R0; ++r) {
-            const float4 a = in ? src[(long long)r * (N / R0) * k.ny / 2] : make_float4(0.f, 0.f, 0.f, 0.f);
-            v[r] = c2{pack2(a.x, a.z), pack2(a.y, a.w)};
-        }
-    }
+            for (int r = 0; r < R0; ++r) {
+                const float4 a = in ? src[(long long)r * (N / R0) * k.ny / 2] : make_float4(0.f, 0.f, 0.f, 0.f);
+                V[m * R0 + r] = c2{pack2(a.x, a.z), pack2(a.y, a.w)};
+            }
+        });
     {
         const float2* gf = c == 0 ? k.Fx : k.Bx;
         for (int i = t; i < N; i += NT) {
             const float2 w = k.tw_x[i], f = gf[i];
-            const float kx = k.kx[i];
             tw[i] = make_float4(w.x, w.x, w.y, w.y);
-            tx[i] = make_float4(f.x * sc, f.x * sc, f.y * sc, f.y * sc);
-            tk[i] = kx * kx;
+            tx[i] = make_float4(f.x, f.x, f.y, f.y);
+            tk[i] = k.kx[i];
         }
     }
     __syncthreads();
-    F::template first<false>(buf, t, v);
-    F::template finish<false>(TwAll<N>{tw}, buf, t, V);
+    F::template first<false>(W, buf, t, V);
+    F::template finish<false>(W, buf, t, V);
+    F::turn(buf, t, V);
 
-    int pl, jl, pe, je;
-    const bool actl = F::template task<F::NST - 1>(t, pl, jl);
-    const bool acte = I::template task<I::NST - 1>(t, pe, je);
     const float kzv = k.kz[kz];
-    // rows of this thread's pair (the same in every stage of a pencil-fast
-    // tile): wavenumbers and y shifts
-    const int y = min(y0 + 2 * pl, k.ny - 2);
-    const float ka = k.ky[y], kb = k.ky[y + 1];
-    const f2 kyz = pack2(ka * ka + kzv * kzv, kb * kb + kzv * kzv);
+    const float kz2 = kzv * kzv;
+    // rows of this thread's pair: wavenumbers and y shifts
+    const int yr = min(y, k.ny - 2);
+    const f2 ky = pack2(k.ky[yr], k.ky[yr + 1]);
     const float2* gy = c == 1 ? k.Fy : k.By;
-    const float2 ya = gy[y], yb = gy[y + 1], zz = (c == 2 ? k.Fz : k.Bz)[kz];
+    const float2 ya = gy[yr], yb = gy[yr + 1], zz = (c == 2 ? k.Fz : k.Bz)[kz];
 
     // seven fields: per axis |k|^-1 and |k|, on the x axis also the identity
     // operator (the other two have one-axis multipliers and are formed elsewhere)
@@ -420,45 +413,47 @@ __global__ void __launch_bounds__(mp_threads(N), mp_blocks(N)) k_mp(KP k, int kz
         if (parts == 3 && ax != part) continue;
         const int d = c == 0 ? (ax == 0 ? 0 : ax == 1 ? 5 : 3) : c == 1 ? (ax == 0 ? 6 : ax == 1 ? 1 : 7)
                                                                         : (ax == 0 ? 4 : ax == 1 ? 8 : 2);
-        if (actl) {
-            f2 cx = ax == 1 ? pack2(ya.x * sc, yb.x * sc) : pack2(zz.x * sc, zz.x * sc);
-            f2 cy = ax == 1 ? pack2(ya.y * sc, yb.y * sc) : pack2(zz.y * sc, zz.y * sc);
+        if (act) {
+            const f2 cx = ax == 1 ? pack2(ya.x, yb.x) : pack2(zz.x, zz.x);
+            const f2 cy = ax == 1 ? pack2(ya.y, yb.y) : pack2(zz.y, zz.y);
+            F::template each<0>(j, [&](int m, int i0) {
 #pragma unroll
-            for (int r = 0; r < RL; ++r) {
-                const int i = jl + r * (N / RL);
-                f2 mx = cx, my = cy;
-                if (ax == 0) {
-                    const float4 m = tx[i];
-                    mx = pack2(m.x, m.y);
-                    my = pack2(m.z, m.w);
+                for (int r = 0; r < R0; ++r) {
+                    const int i = i0 + r * (N / R0);
+                    f2 mx = cx, my = cy;
+                    if (ax == 0) {
+                        const float4 T = tx[i];
+                        mx = pack2(T.x, T.y);
+                        my = pack2(T.z, T.w);
+                    }
+                    f2 s = pack2(sc, sc);
+                    if (jj != 1) {
+                        const f2 kx = pack2(tk[i], tk[i]);
+                        const float2 s2 = unpack2(fma_(kx, kx, ky * ky) + pack2(kz2, kz2));
+                        // the reference sets |k|^2 = 1e-10 at DC (cu:74)
+                        const float a = fmaxf(s2.x, 1e-10f), b = fmaxf(s2.y, 1e-10f);
+                        // |k|^-1 and |k| from the hardware reciprocal square root
+                        // (~2 ulp): far below the FP32 transforms' own rounding
+                        f2 ap = pack2(rsqrtf(a), rsqrtf(b));
+                        if (jj == 2) ap = ap * pack2(a, b);
+                        s = ap * s;
+                    }
+                    v[m * R0 + r] = cmul_tw<false>(V[m * R0 + r], mx * s, my * s);
                 }
-                if (jj != 1) {
-                    const float kx2 = tk[i];
-                    const float2 s2 = unpack2(pack2(kx2, kx2) + kyz);
-                    // the reference sets |k|^2 = 1e-10 at DC (cu:74)
-                    const float a = fmaxf(s2.x, 1e-10f), b = fmaxf(s2.y, 1e-10f);
-                    // |k|^-1 and |k| from the hardware reciprocal square root
-                    // (~2 ulp): far below the FP32 transforms' own rounding
-                    f2 ap = pack2(rsqrtf(a), rsqrtf(b));
-                    if (jj == 2) ap = ap * pack2(a, b);
-                    mx = mx * ap;
-                    my = my * ap;
-                }
-                v[r] = cmul_tw<false>(V[r], mx, my);
-            }
+            });
         }
         __syncthreads();  // the previous transform's last reads of the exchange
-        I::template first<true>(buf, t, v);
-        I::template finish<true>(TwAll<N>{tw}, buf, t, v);
-        const int ye = y0 + 2 * pe;
-        if (acte && ye < k.ny) {
-            float4* dst = reinterpret_cast<float4*>(k.G[3 * d + jj] + spec(k, kz, je, ye));
+        F::template first<true>(W, buf, t, v);
+        F::template finish<true>(W, buf, t, v);
+        if (act && in)
+            F::template each<F::LAST>(j, [&](int m, int i) {
+                float4* dst = reinterpret_cast<float4*>(k.G[3 * d + jj] + spec(k, kz, i, y));
 #pragma unroll
-            for (int r = 0; r < R0; ++r) {
-                const float2 x = unpack2(v[r].x), q = unpack2(v[r].y);
-                dst[(long long)r * (N / R0) * k.ny / 2] = make_float4(x.x, q.x, x.y, q.y);
-            }
-        }
+                for (int r = 0; r < RL; ++r) {
+                    const float2 x = unpack2(v[m * RL + r].x), q = unpack2(v[m * RL + r].y);
+                    dst[(long long)r * (N / RL) * k.ny / 2] = make_float4(x.x, q.x, x.y, q.y);
+                }
+            });
     }
 }
 
@@ -529,7 +524,7 @@ size_t smem_cy(const KP& k, int L, bool ydv, bool rt)
 size_t smem_mx(const KP& k, int P, bool rt)
 {
     if (!rt) return mp_smem(k.nx);
-    const int nbuf = k.px.nst > 2 ? 2 : 1;
+    const int nbuf = k.px.q.nst > 2 ? 2 : 1;
     return sizeof(float2) * (3 * k.nx + k.nx * P + nbuf * (k.nx + k.nx / 16) * P + 2 * P) + sizeof(float) * (k.nx + P);
 }
 

@@ -117,7 +117,7 @@ __global__ void __launch_bounds__(kThreads) k_vy(KP k, int P)
         fft_rt<kPencil, false>(k.py, tw, A, B, Qp, 1, Qp, load, store);
         float2* X1 = Zf == A ? B : A;
         float* D = reinterpret_cast<float*>(fft_out_buf(k.py, X1, Zf));  // [n][P]
-        auto load_i = [&](int q, int i) -> float2 { return cmul(Zf[i * Qp + q], cscale(tF[i], inv_n)); };
+        auto load_i = [&](int q, int i) -> float2 { return cmul_m(Zf[i * Qp + q], cscale(tF[i], inv_n)); };
         auto store_i = [&](int q, int i, float2 v) {
             D[i * P + 2 * q] = v.x;
             D[i * P + 2 * q + 1] = v.y;
@@ -270,7 +270,7 @@ __global__ void __launch_bounds__(kThreads) k_vx(KP k, int P)
         fft_rt<kPencil, false>(k.px, tw, A, B, Qp, 1, Qp, load, store);
         float2* X1 = Zf == A ? B : A;
         float* D = reinterpret_cast<float*>(fft_out_buf(k.px, X1, Zf));  // [n][P]
-        auto load_i = [&](int q, int i) -> float2 { return cmul(Zf[i * Qp + q], cscale(tF[i], inv_n)); };
+        auto load_i = [&](int q, int i) -> float2 { return cmul_m(Zf[i * Qp + q], cscale(tF[i], inv_n)); };
         auto store_i = [&](int q, int i, float2 v) {
             D[i * P + 2 * q] = v.x;
             D[i * P + 2 * q + 1] = v.y;
@@ -317,176 +317,288 @@ __global__ void __launch_bounds__(kThreads) k_vx(KP k, int P)
 // Compiled form of both velocity kernels.  AX = 1 (k_vy's job): the y
 // derivatives of sxy (+), syy (-), syz (+) with their C-PML terms added to R.
 // AX = 0 (k_vx's): the x derivatives of sxx (-), sxy (+), sxz (+), their C-PML
-// terms and the velocity update (cu:1018-1101).  A block owns 16 consecutive z
-// of one line and takes the three fields one after another.
+// terms and the velocity update (cu:1018-1101).  A block owns consecutive z of
+// one line: the first blocks of a line 2 PP z of the first two fields, which
+// share one complex transform (two_shift), z and z + 1 in a packed pair; the
+// others 4 PP z of the third, z + 1 the imaginary part of z, two such pencils in
+// a pair.
 //
-// Four consecutive z of a field are two complex pencils, (z + 2) i added to z
-// and (z + 3) i to z + 1: one multiplier serves all, a 16-byte load IS the
-// packed pair, and what the inverse's last stage leaves in a thread is four
-// consecutive z of the derivative, so the epilogue reads and writes the other
-// arrays 16 bytes at a time straight from registers.  Per field: two exchanges
-// through shared memory (forward and inverse, reversed radices: nothing is
-// exchanged at the multiplication).  The kernels they replace kept every
-// derivative in shared memory for a scalar epilogue and ran at 55 % issue
-// between barriers.
+// The derivatives go back to the exchange for the epilogue, a loop in which
+// consecutive lanes take consecutive z, two cells at a time with all their loads
+// ahead of their stores.  (As straight code on the registers the inverse ends in
+// the epilogue was four fifths of the kernel's instructions and 83 MB of the
+// library.)  The kernels they replace ran scalar transforms at 55 % issue between
+// barriers.
 constexpr int dv_threads(int n, int pp) { return warps_up(pp * pair_tasks(n)); }
 constexpr size_t dv_smem(int n, int pp) { return 16 * ((size_t)pp * pair_slots(n) + 2 * (size_t)n); }
 // Blocks per SM the registers are sized for: a thread holds the pair's
-// butterfly (4 registers a point) and the loads of the epilogue.
+// butterflies (4 registers a point) and the loads of the epilogue.
 // Warps come in fours, one per scheduler, or a scheduler's registers are split
 // more ways than the others'.
 constexpr int dv_blocks(int n, int pp)
 {
-    const int warps = dv_threads(n, pp) / 32, regs = pair_rmax(n) >= 10 ? 128 : 96;
-    int b = 65536 / (regs * dv_threads(n, pp));
+    const int warps = dv_threads(n, pp) / 32;
+    int b = 65536 / (128 * dv_threads(n, pp));
     const int m = (int)(220 * 1024 / (dv_smem(n, pp) + 1024));
     if (m < b) b = m;
     while (b > 1 && b * warps % 4) --b;
     return b < 1 ? 1 : b;
 }
 
-template <bool V4>
-__device__ __forceinline__ float4 ld4(const float* p, int left)  // `left` values of the row remain (even)
+// W = 2 or 4 consecutive z of a row of which `left` remain (even): 8-byte
+// accesses, or one of 16 (v4: the rows are 16-byte aligned).
+template <int W>
+__device__ __forceinline__ void ldz(float* o, const float* p, int left, bool v4)
 {
-    if constexpr (V4) return left > 0 ? *reinterpret_cast<const float4*>(p) : make_float4(0.f, 0.f, 0.f, 0.f);
-    const float2 a = left > 0 ? *reinterpret_cast<const float2*>(p) : make_float2(0.f, 0.f);
-    const float2 b = left > 2 ? *reinterpret_cast<const float2*>(p + 2) : make_float2(0.f, 0.f);
-    return make_float4(a.x, a.y, b.x, b.y);
-}
-template <bool V4>
-__device__ __forceinline__ void st4(float* p, int left, float4 v)
-{
-    if constexpr (V4) {
-        if (left > 0) *reinterpret_cast<float4*>(p) = v;
+    if (W == 4 && v4) {
+        const float4 a = left > 0 ? *reinterpret_cast<const float4*>(p) : make_float4(0.f, 0.f, 0.f, 0.f);
+        o[0] = a.x; o[1] = a.y; o[W - 2] = a.z; o[W - 1] = a.w;
     } else {
-        if (left > 0) *reinterpret_cast<float2*>(p) = make_float2(v.x, v.y);
-        if (left > 2) *reinterpret_cast<float2*>(p + 2) = make_float2(v.z, v.w);
+#pragma unroll
+        for (int u = 0; u < W; u += 2) {
+            const float2 a = left > u ? *reinterpret_cast<const float2*>(p + u) : make_float2(0.f, 0.f);
+            o[u] = a.x; o[u + 1] = a.y;
+        }
+    }
+}
+template <int W>
+__device__ __forceinline__ void stz(float* p, int left, bool v4, const float* v)
+{
+    if (W == 4 && v4) {
+        if (left > 0) *reinterpret_cast<float4*>(p) = make_float4(v[0], v[1], v[W - 2], v[W - 1]);
+    } else {
+#pragma unroll
+        for (int u = 0; u < W; u += 2)
+            if (left > u) *reinterpret_cast<float2*>(p + u) = make_float2(v[u], v[u + 1]);
     }
 }
 
 __device__ __forceinline__ void prefetch_line(const float* p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
 
-template <int N, int PP, int AX, bool V4>
+// A velocity field's part of the epilogue: W z from z on at index i of the line;
+// back: the shift is backward, the C-PML profile the half-point average.
+template <int W>
+struct DvCell {
+    float r[W], o[W], w[W], q[W];
+    int ip, is;
+    bool on, slab;
+};
+template <int N, int AX, int W>
+struct DvEpi {
+    const KP& k;
+    int line, base, stride;
+    bool lin, v4;  // lin: cells of this line are updated (k_vx), or have C-PML terms (k_vy)
+    float *R, *vel, *ph;
+    const float *ri, *pa, *pb;
+    __device__ __forceinline__ DvEpi(const KP& k_, int f, bool back, int line_)
+        : k(k_), line(line_), v4(k_.nz % 4 == 0), R(k_.R[f]), vel(k_.v[f]), ph(k_.php[AX ? 3 * f + 1 : 3 * f]),
+          ri(k_.rinv[f]), pa(AX ? (back ? k_.ayh : k_.ay) : (back ? k_.axh : k_.ax)),
+          pb(AX ? (back ? k_.byh : k_.by) : (back ? k_.bxh : k_.bx))
+    {
+        stride = AX ? k.nz : k.ny * k.nz;
+        base = AX ? line * k.ny * k.nz : line * k.nz;
+        lin = AX ? line < k.nx - 1 : line < k.ny - 1;
+    }
+    __device__ __forceinline__ int slab_at(int i, int z) const { return AX ? slab_y(k, line, i, z) : slab_x(k, i, line, z); }
+    __device__ __forceinline__ void prefetch(int i, int z) const
+    {
+        const int ip = base + i * stride + z;
+        prefetch_line(R + ip);
+        if (AX == 0) {
+            prefetch_line(vel + ip);
+            prefetch_line(ri + ip);
+        }
+        if (lin && in_slab(i, N, k.pml)) prefetch_line(ph + slab_at(i, z));
+    }
+    __device__ __forceinline__ void load(DvCell<W>& c, bool ok, int i, int z) const
+    {
+        const int left = k.nz - z;
+        const bool in = lin && i < N - 1;
+        c.on = ok && left > 0 && (AX || in);
+        c.slab = c.on && in && in_slab(i, N, k.pml);
+        c.ip = base + i * stride + z;
+        c.is = c.slab ? slab_at(i, z) : 0;
+        ldz<W>(c.r, R + c.ip, c.on ? left : 0, v4);
+        if (AX == 0) {
+            ldz<W>(c.o, vel + c.ip, c.on ? left : 0, v4);
+            ldz<W>(c.w, ri + c.ip, c.on ? left : 0, v4);
+        }
+        ldz<W>(c.q, ph + c.is, c.slab ? left : 0, v4);
+    }
+    __device__ __forceinline__ void store(DvCell<W>& c, int i, int z, float* d) const
+    {
+        const int left = k.nz - z;
+        const float dt = k.dt;
+        if (!c.on) return;
+        if (AX == 1) {
+#pragma unroll
+            for (int u = 0; u < W; ++u) c.r[u] += d[u];
+        }
+        if (c.slab) {
+            const float a = pa[i], b = pb[i];
+#pragma unroll
+            for (int u = 0; u < W; ++u)
+                if (u < left - 1) {  // all but the last plane
+                    c.q[u] = pml_step(c.q[u], dt, a, b, d[u]);
+                    (AX ? c.r : d)[u] += c.q[u];
+                }
+            stz<W>(ph + c.is, left, v4, c.q);
+        }
+        if (AX == 1) {
+            stz<W>(R + c.ip, left, v4, c.r);
+        } else {
+#pragma unroll
+            for (int u = 0; u < W; ++u)
+                if (u < left - 1) c.o[u] = fmaf(dt * c.w[u], d[u] + c.r[u], c.o[u]);
+            stz<W>(vel + c.ip, left, v4, c.o);
+        }
+    }
+};
+
+template <int N, int PP, int AX>
 __global__ void __launch_bounds__(dv_threads(N, PP), dv_blocks(N, PP)) k_dv(KP k)
 {
-    using F = PairFFT<N, PP, true, false>;
-    using I = PairFFT<N, PP, true, true>;
-    constexpr int NT = dv_threads(N, PP), RM = pair_rmax(N), RL = F::RL, R0 = F::R0;
+    using F = PairFFT<N, PP, true>;
+    constexpr int NT = dv_threads(N, PP), R0 = F::R0;
+    static_assert(NT <= 1024, "threads of a block");
     extern __shared__ float4 smem4[];
     f2* buf = reinterpret_cast<f2*>(smem4);
     float4* tw = smem4 + PP * pair_slots(N);
     float4* tf = tw + N;  // forward shift over n, doubled like the twiddles; the backward one is (-F.x, F.y)
-    if (AX == 1 && blockIdx.x + blockIdx.y + blockIdx.z == 0 && threadIdx.x == 0) *k.d_it += 1;  // step counter
-    const int t = threadIdx.x, nz = k.nz, pml = k.pml;
+    if (AX == 1 && blockIdx.x + blockIdx.y == 0 && threadIdx.x == 0) *k.d_it += 1;  // step counter
+    const int t = threadIdx.x, nz = k.nz;
     const int line = blockIdx.y;  // x (AX = 1) or y
     const int stride = AX ? nz : k.ny * nz;
-    const float dt = k.dt;
-    // cells of this line are updated (k_vx), or have C-PML terms (k_vy)
-    const bool lin = AX ? line < k.nx - 1 : line < k.ny - 1;
-    const float* pa = AX ? k.ay : k.ax;
-    const float* pb = AX ? k.by : k.bx;
-    const float* pah = AX ? k.ayh : k.axh;
-    const float* pbh = AX ? k.byh : k.bxh;
-    int p0, j0, pl, jl, pe, je;
-    const bool act0 = F::template task<0>(t, p0, j0);
-    const bool actl = F::template task<F::NST - 1>(t, pl, jl);
-    const bool acte = I::template task<I::NST - 1>(t, pe, je);
-    const int zl = blockIdx.x * (4 * PP) + 4 * p0, ze = blockIdx.x * (4 * PP) + 4 * pe;
-    const int f = blockIdx.z;
-    {
-        // the field, its target, and the one with the backward shift (whose
-        // C-PML profile is the half-point average)
-        const float* src = k.s[AX ? (f == 0 ? 3 : f == 1 ? 1 : 5) : (f == 0 ? 0 : f == 1 ? 3 : 4)];
-        const bool back = f == (AX ? 1 : 0);
-        c2 v[RM];
-        if (act0) {
-            const int b0 = (AX ? line * k.ny * nz : line * nz) + j0 * stride + zl;
-#pragma unroll
-            for (int r = 0; r < R0; ++r) {
-                const float4 a = ld4<V4>(src + b0 + r * (N / R0) * stride, nz - zl);
-                v[r] = c2{pack2(a.x, a.y), pack2(a.z, a.w)};
-            }
+    const int base = AX ? line * k.ny * nz : line * nz;
+    const int pairs = (nz + 2 * PP - 1) / (2 * PP);  // blocks of the first two fields
+    int p, j;
+    const bool act = F::task(t, p, j);
+    c2 v[F::RM];
+    auto tables = [&] {  // behind the loads in flight (read after the exchange's barrier)
+        const float2* gtw = AX ? k.tw_y : k.tw_x;
+        const float2* gf = AX ? k.Fy : k.Fx;
+        constexpr float inv_n = 1.0f / N;
+        for (int i = threadIdx.x; i < N; i += NT) {
+            const float2 w = gtw[i], f = gf[i];
+            tw[i] = make_float4(w.x, w.x, w.y, w.y);
+            tf[i] = make_float4(f.x * inv_n, f.x * inv_n, f.y * inv_n, f.y * inv_n);
         }
-        float* __restrict__ ph = k.php[AX ? 3 * f + 1 : 3 * f];
-        float* __restrict__ R = k.R[f];
-        float* __restrict__ vel = k.v[f];
-        const float* __restrict__ ri = k.rinv[f];
-        const int left = nz - ze;
-        const int be = (AX ? line * k.ny * nz : line * nz) + ze;
-        // the epilogue's operands start their way from HBM to L2 now
-        if (acte && left > 0) {
+        if (F::SYNC0) __syncthreads();
+    };
+    const TwAll<N> W{tw};
+    if (blockIdx.x < pairs) {
+        const int z0 = blockIdx.x * 2 * PP, z = z0 + 2 * p, left = nz - z;
+        const float* sa = k.s[AX ? 3 : 0] + base + z;
+        const float* sb = k.s[AX ? 1 : 3] + base + z;
+        if (act)
+            F::template each<0>(j, [&](int m, int i) {
 #pragma unroll
-            for (int r = 0; r < R0; ++r) {
-                const int i = je + r * (N / R0), ip = be + i * stride;
-                prefetch_line(R + ip);
-                if (AX == 0) {
-                    prefetch_line(vel + ip);
-                    prefetch_line(ri + ip);
+                for (int r = 0; r < R0; ++r) {
+                    const int at = (i + r * (N / R0)) * stride;
+                    float a[2], b[2];
+                    ldz<2>(a, sa + at, left, false);
+                    ldz<2>(b, sb + at, left, false);
+                    v[m * R0 + r] = c2{pack2(a[0], a[1]), pack2(b[0], b[1])};
                 }
-                if (lin && in_slab(i, N, pml)) prefetch_line(ph + (AX ? slab_y(k, line, i, ze) : slab_x(k, i, line, ze)));
-            }
+            });
+        // k_vy: sxy forward, syy backward; k_vx: sxx backward, sxy forward
+        const DvEpi<N, AX, 2> ea(k, 0, AX == 0, line), eb(k, 1, AX == 1, line);
+        // the epilogue's operands start their way from HBM to L2 now
+        for (int i = t; i < 2 * N; i += NT) {
+            const int zp = min(z0 + (i & 1 ? 2 * PP - 1 : 0), nz - 1);
+            ea.prefetch(i / 2, zp);
+            eb.prefetch(i / 2, zp);
         }
-        {  // tables, behind the loads in flight (read after the exchange's barrier)
-            const float2* gtw = AX ? k.tw_y : k.tw_x;
-            const float2* gf = AX ? k.Fy : k.Fx;
-            constexpr float inv_n = 1.0f / N;
-            for (int i = threadIdx.x; i < N; i += NT) {
-                const float2 w = gtw[i], f = gf[i];
-                tw[i] = make_float4(w.x, w.x, w.y, w.y);
-                tf[i] = make_float4(f.x * inv_n, f.x * inv_n, f.y * inv_n, f.y * inv_n);
-            }
-        }
-        F::template first<false>(buf, t, v);
-        F::template finish<false>(TwAll<N>{tw}, buf, t, v);
-        if (actl) {
-#pragma unroll
-            for (int r = 0; r < RL; ++r) {
-                const float4 m = tf[jl + r * (N / RL)];
-                f2 mx = pack2(m.x, m.y);
-                const f2 my = pack2(m.z, m.w);
-                if (back) mx = neg_(mx);
-                v[r] = cmul_tw<false>(v[r], mx, my);
-            }
-        }
+        tables();
+        F::template first<false>(W, buf, t, v);
+        F::template finish<false>(W, buf, t, v);
+        F::keep(buf, t, v);
         __syncthreads();
-        I::template first<true>(buf, t, v);
-        I::template finish<true>(TwAll<N>{tw}, buf, t, v);
-        if (!acte || left <= 0) return;
+        if (act)
+            F::template each<0>(j, [&](int m, int i0) {
 #pragma unroll
-        for (int r = 0; r < R0; ++r) {
-            const int i = je + r * (N / R0);
-            const int ip = be + i * stride;
-            const bool in = lin && i < N - 1;
-            if (AX == 0 && !in) continue;
-            const float2 dx = unpack2(v[r].x), dy = unpack2(v[r].y);
-            float d[4] = {dx.x, dx.y, dy.x, dy.y};
-            const float4 rr = ld4<V4>(R + ip, left);
-            float4 vv, wi;
-            if (AX == 0) {
-                vv = ld4<V4>(vel + ip, left);
-                wi = ld4<V4>(ri + ip, left);
+                for (int r = 0; r < R0; ++r) {
+                    const int i = i0 + r * (N / R0);
+                    const c2 z = F::ld(buf + F::slot(p, i)), c = F::ld(buf + F::slot(p, i ? N - i : 0));
+                    const float4 f = tf[i];
+                    // two_shift, sgn = 1 (k_vy) or -1
+                    const f2 fx = pack2(AX ? f.x : -f.x, AX ? f.x : -f.x), nx = pack2(AX ? -f.x : f.x, AX ? -f.x : f.x);
+                    const f2 fy = pack2(f.z, f.z), ny = pack2(-f.z, -f.z);
+                    v[m * R0 + r] = c2{fma_(fx, c.x, ny * z.y), fma_(nx, c.y, fy * z.x)};
+                }
+            });
+        __syncthreads();
+        F::template first<true>(W, buf, t, v);
+        F::template finish<true>(W, buf, t, v);
+        F::keep(buf, t, v);
+        __syncthreads();
+#pragma unroll 1
+        for (int w = t; w < N * PP; w += 2 * NT) {
+            DvCell<2> a[2], b[2];
+#pragma unroll
+            for (int u = 0; u < 2; ++u) {
+                const int i = (unsigned)(w + u * NT) / PP, zc = z0 + 2 * ((w + u * NT) % PP);
+                ea.load(a[u], i < N, i, zc);
+                eb.load(b[u], i < N, i, zc);
             }
-            if (in && in_slab(i, N, pml)) {
-                const int is = (AX ? slab_y(k, line, i, ze) : slab_x(k, i, line, ze));
-                const float a = back ? pah[i] : pa[i], b = back ? pbh[i] : pb[i];
-                const float4 o = ld4<V4>(ph + is, left);
-                float q[4] = {o.x, o.y, o.z, o.w};
 #pragma unroll
-                for (int u = 0; u < 4; ++u)
-                    if (u < left - 1) {  // all but the last plane
-                        q[u] = q[u] + dt * (-a * q[u] - b * d[u]);
-                        d[u] += q[u];
-                    }
-                st4<V4>(ph + is, left, make_float4(q[0], q[1], q[2], q[3]));
+            for (int u = 0; u < 2; ++u) {
+                const int i = (unsigned)(w + u * NT) / PP, q = (w + u * NT) % PP;
+                if (i >= N) break;
+                const c2 d = F::ld(buf + F::slot(q, i));
+                const float2 x = unpack2(d.x), y = unpack2(d.y);
+                float da[2] = {x.x, x.y}, db[2] = {y.x, y.y};
+                ea.store(a[u], i, z0 + 2 * q, da);
+                eb.store(b[u], i, z0 + 2 * q, db);
             }
-            if (AX == 1) {
-                st4<V4>(R + ip, left, make_float4(rr.x + d[0], rr.y + d[1], rr.z + d[2], rr.w + d[3]));
-            } else {
-                const float o[4] = {vv.x, vv.y, vv.z, vv.w}, w[4] = {wi.x, wi.y, wi.z, wi.w}, q[4] = {rr.x, rr.y, rr.z, rr.w};
-                float n[4];
+        }
+    } else {
+        const int z0 = (blockIdx.x - pairs) * 4 * PP, z = z0 + 4 * p, left = nz - z;
+        const float* src = k.s[AX ? 5 : 4] + base + z;
+        const DvEpi<N, AX, 4> e(k, 2, false, line);
+        if (act)
+            F::template each<0>(j, [&](int m, int i) {
 #pragma unroll
-                for (int u = 0; u < 4; ++u) n[u] = u < left - 1 ? o[u] + dt * w[u] * (d[u] + q[u]) : o[u];
-                st4<V4>(vel + ip, left, make_float4(n[0], n[1], n[2], n[3]));
+                for (int r = 0; r < R0; ++r) {
+                    float a[4];
+                    ldz<4>(a, src + (i + r * (N / R0)) * stride, left, e.v4);
+                    v[m * R0 + r] = c2{pack2(a[0], a[2]), pack2(a[1], a[3])};
+                }
+            });
+        for (int i = t; i < 3 * N; i += NT) e.prefetch(i / 3, min(z0 + (i % 3 * (4 * PP - 1)) / 2, nz - 1));
+        tables();
+        F::template first<false>(W, buf, t, v);
+        F::template finish<false>(W, buf, t, v);
+        F::turn(buf, t, v);
+        if (act)
+            F::template each<0>(j, [&](int m, int i) {
+#pragma unroll
+                for (int r = 0; r < R0; ++r) {
+                    const float4 f = tf[i + r * (N / R0)];
+                    v[m * R0 + r] = cmul_m(v[m * R0 + r], pack2(f.x, f.y), pack2(f.z, f.w));
+                }
+            });
+        __syncthreads();
+        F::template first<true>(W, buf, t, v);
+        F::template finish<true>(W, buf, t, v);
+        F::keep(buf, t, v);
+        __syncthreads();
+#pragma unroll 1
+        for (int w = t; w < N * PP; w += 2 * NT) {
+            DvCell<4> a[2];
+#pragma unroll
+            for (int u = 0; u < 2; ++u) {
+                const int i = (unsigned)(w + u * NT) / PP;
+                e.load(a[u], i < N, i, z0 + 4 * ((w + u * NT) % PP));
+            }
+#pragma unroll
+            for (int u = 0; u < 2; ++u) {
+                const int i = (unsigned)(w + u * NT) / PP, q = (w + u * NT) % PP;
+                if (i >= N) break;
+                const c2 c = F::ld(buf + F::slot(q, i));
+                const float2 x = unpack2(c.x), y = unpack2(c.y);
+                float d[4] = {x.x, y.x, x.y, y.y};
+                e.store(a[u], i, z0 + 4 * q, d);
             }
         }
     }
@@ -502,13 +614,12 @@ bool dv_launch<QVTI_PART>(const KP& k, int ax, int P, cudaStream_t st)
 {
     return dispatch_len(ax ? k.ny : k.nx, [&](auto NN) {
         constexpr int N = decltype(NN)::value;
-        const dim3 grid(cdiv(k.nz, P), ax ? k.nx : k.ny, 3);
+        const dim3 grid(cdiv(k.nz, P) + cdiv(k.nz, 2 * P), ax ? k.nx : k.ny);
         auto go = [&](auto AX) {
             constexpr int ax_ = decltype(AX)::value;
-            const size_t sm = dv_smem(N, P / 4);
-            if (k.nz % 4) k_dv<N, 8, ax_, false><<<grid, dv_threads(N, 8), sm, st>>>(k);  // rows only 8-byte aligned
-            else if (P == 16) k_dv<N, 4, ax_, true><<<grid, dv_threads(N, 4), sm, st>>>(k);
-            else k_dv<N, 8, ax_, true><<<grid, dv_threads(N, 8), sm, st>>>(k);
+            const size_t sm = dv_smem(N, P / 2);
+            if (P == 16) k_dv<N, 8, ax_><<<grid, dv_threads(N, 8), sm, st>>>(k);
+            else k_dv<N, 16, ax_><<<grid, dv_threads(N, 16), sm, st>>>(k);
         };
         if (ax) {
             go(IntC<1>{});
@@ -523,21 +634,20 @@ bool dv_configure<QVTI_PART>(SmemLimit& lim)
     for (int n : kMyLengths)
         dispatch_len(n, [&](auto NN) {
             constexpr int N = decltype(NN)::value;
-            lim.set((const void*)k_dv<N, 8, 1, true>);
-            lim.set((const void*)k_dv<N, 4, 1, true>);
-            lim.set((const void*)k_dv<N, 8, 1, false>);
-            if constexpr (N >= kMinLong) {
-                lim.set((const void*)k_dv<N, 8, 0, true>);
-                lim.set((const void*)k_dv<N, 4, 0, true>);
-                lim.set((const void*)k_dv<N, 8, 0, false>);
-            }
+            auto set = [&](auto AX) {
+                constexpr int ax = decltype(AX)::value;
+                lim.set((const void*)k_dv<N, 8, ax>);
+                lim.set((const void*)k_dv<N, 16, ax>);
+            };
+            set(IntC<1>{});
+            if constexpr (N >= kMinLong) set(IntC<0>{});
         });
     return false;
 }
 
 #if QVTI_PART == 0
 // rt: the runtime kernels' layout.
-size_t smem_vyx(int n, int P, bool rt) { return rt ? sizeof(float2) * (2 * n + 2 * (n + n / 16) * P) : dv_smem(n, P / 4); }
+size_t smem_vyx(int n, int P, bool rt) { return rt ? sizeof(float2) * (2 * n + 2 * (n + n / 16) * P) : dv_smem(n, P / 2); }
 
 void launch_vy(const KP& k, int P, bool rt, cudaStream_t st)
 {

@@ -155,7 +155,7 @@ __global__ void __launch_bounds__(kQdThreads) k_qd(const __grid_constant__ QdArg
     // x forward, |k|^pw T(k_axis) / ntp, x inverse: P consecutive y of one kz
     {
         const int ps = layout(0), chunks = (ny + P - 1) / P, tiles = chunks * a.nkz;
-        float2* tT = B + (a.pl[0].nst > 2 ? P * ps : 0);  // the shift over the axis it varies on
+        float2* tT = B + (a.pl[0].q.nst > 2 ? P * ps : 0);  // the shift over the axis it varies on
         float* tk = reinterpret_cast<float*>(tT + max(nx, P));
         float* tky = tk + nx;
         for (int i = t; i < nx; i += kQdThreads) {
@@ -231,7 +231,7 @@ size_t qd_smem(const QdArgs& a, int P)
 {
     size_t m = 0;
     for (int ax = 0; ax < 3; ++ax) {
-        const size_t n = a.n[ax], ps = n + n / 16, nb = a.pl[ax].nst > 2 ? 3 : 2;
+        const size_t n = a.n[ax], ps = n + n / 16, nb = a.pl[ax].q.nst > 2 ? 3 : 2;
         size_t b = sizeof(float2) * (n + nb * P * ps);
         if (ax == 0) b += sizeof(float2) * std::max<size_t>(n, P) + sizeof(float) * (n + P);
         m = std::max(m, b);

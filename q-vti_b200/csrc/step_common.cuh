@@ -21,6 +21,12 @@ __device__ __forceinline__ int cell(const KP& k, int x, int y, int z) { return (
 __device__ __forceinline__ int spec(const KP& k, int kz, int x, int y) { return (kz * k.nx + x) * k.ny + y; }
 __device__ __forceinline__ bool in_slab(int i, int n, int pml) { return i < pml || i >= n - pml; }
 
+// One step of a C-PML memory variable q with the term d of its axis.
+__device__ __forceinline__ float pml_step(float q, float dt, float a, float b, float d)
+{
+    return fmaf(dt, fmaf(-a, q, -(b * d)), q);
+}
+
 __device__ __forceinline__ void load_table(float2* s, const float2* g, int n)
 {
     for (int i = threadIdx.x; i < n; i += blockDim.x) s[i] = g[i];
@@ -105,7 +111,7 @@ static bool dispatch_len(int n, F&& f)
 inline int rt_threads(const FftPlan& p, int pencils)
 {
     int m = 0;
-    for (int s = 0; s < p.nst; ++s) m = p.n / p.rad[s] > m ? p.n / p.rad[s] : m;
+    for (int s = 0; s < p.q.nst; ++s) m = p.n / p.q.rad(s) > m ? p.n / p.q.rad(s) : m;
     const int t = (m * pencils + 31) / 32 * 32;
     return t < kThreads ? t : kThreads;
 }

@@ -176,7 +176,7 @@ __global__ void k_deriv1d(KP k, int axis, int fwd, const float* in, float* out, 
     fft_run<true, false>(pl, tw, A, B, Qp, 1, Qp, load, store);
     float2* X1 = Zf == A ? B : A;
     const float inv_n = 1.0f / n;
-    auto load_i = [&](int q, int i) -> float2 { return cmul(Zf[i * Qp + q], cscale(T[i], inv_n)); };
+    auto load_i = [&](int q, int i) -> float2 { return cmul_m(Zf[i * Qp + q], cscale(T[i], inv_n)); };
     auto store_i = [&](int q, int i, float2 v) {
         const long long p0 = pen0 + 2 * q, p1 = p0 + 1;
         if (p0 < npen) out[addr(p0, i)] = v.x;
@@ -278,7 +278,7 @@ bool ct_length(int n)
 // half of every L1 line it fetched unused and measured 0.21 against 0.15 ms
 // for k_vy, 0.34 against 0.22 for k_vx at 256^3) unless that leaves fewer than
 // two blocks per SM.
-int dv_tile(int nz, int lines) { return nz % 4 || 3ll * cdiv(nz, 32) * lines >= 2 * 148 ? 32 : 16; }
+int dv_tile(int nz, int lines) { return 3ll * cdiv(nz, 64) * lines >= 2 * 148 ? 32 : 16; }
 // The compiled stress kernels take eight rows (half-line accesses, see k_st)
 // unless that leaves fewer than four blocks per SM.
 int st_rows(const KP& k)

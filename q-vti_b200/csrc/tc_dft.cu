@@ -324,7 +324,7 @@ __global__ void __launch_bounds__(kTcThreads, INV ? 5 : 4) k_cy_tc(KP k, int nfi
         for (int q = 0; q < 16; ++q) {
             const float2 a = make_float2(d[2 * q], d[2 * q + 1]);
             const float2 wq = tw[q * j];
-            y[q] = INV ? cmulc(a, wq) : cmul(a, wq);
+            y[q] = INV ? cmulc(a, wq) : cmul_m(a, wq);
         }
         scatter_rows(Ahi, Alo, p, j, y);
         if (!(ok = run_round(tmem, Ahi, Alo, Bhi, Blo, mbar, phase, d))) break;
@@ -339,7 +339,7 @@ __global__ void __launch_bounds__(kTcThreads, INV ? 5 : 4) k_cy_tc(KP k, int nfi
             float2 u[16];
 #pragma unroll
             for (int q = 0; q < 16; ++q)
-                u[q] = cmul(make_float2(d[2 * q], d[2 * q + 1]), cscale(tsh[j + 16 * q], inv_n));
+                u[q] = cmul_m(make_float2(d[2 * q], d[2 * q + 1]), cscale(tsh[j + 16 * q], inv_n));
             put_row(Ahi, Alo, t, u);
             if (!(ok = run_round(tmem, Ahi, Alo, Bi_hi, Bi_lo, mbar, phase, d))) break;
 #pragma unroll
