@@ -382,11 +382,16 @@ size_t step_smem_bytes(const KP& k)
     m = std::max(m, smem_cy(k, T.cy, true, T.rt[3]));
     m = std::max(m, smem_mx(k, T.mx, T.rt[4]));
     m = std::max(m, smem_sigma(k, T.sigma, T.rt[5]));
-    // the grids and tiles that are supported at runtime z lengths are those of
-    // a layout with room for the z derivatives and their tables beside the fields
-    if (T.rt[5])
-        m = std::max(m, smem_sigma(k, T.sigma, true) + sizeof(float2) * 2 * k.nz +
+    // the grids and tiles that are supported at runtime lengths are those of
+    // layouts with a second transform buffer from three radices on, and on the z
+    // axis with room for the z derivatives and their tables beside the fields
+    if (T.rt[4] && k.px.q.radices > 2 && k.px.q.nst == 2)
+        m = std::max(m, smem_mx(k, T.mx, true) + sizeof(float2) * (k.nx + k.nx / 16) * T.mx);
+    if (T.rt[5]) {
+        const size_t more = k.pz.q.radices > 2 && k.pz.q.nst == 2 ? sizeof(float2) * 9 * (T.sigma / 2) * (k.nz + k.nz / 16) : 0;
+        m = std::max(m, smem_sigma(k, T.sigma, true) + more + sizeof(float2) * 2 * k.nz +
                             sizeof(float) * ((size_t)3 * T.sigma * (k.nz + 1) + 4 * k.nz + 4 * T.sigma));
+    }
     return m;
 }
 
