@@ -202,8 +202,9 @@ int qvti_q_derivative(qvti_sim* sim, int axis, int fwd, int power, const float* 
  * 2/3/5/7-smooth, and (ntz/2 + 1)*ntx*nty <= 524288 (4 MiB of scratch, e.g.
  * 96^3 or 64x64x128); larger grids return QVTI_ERR_UNSUPPORTED.  The first
  * call on a device looks up the array's device address (and sets kernel
- * attributes) -- make it before any stream capture.  One cooperative kernel
- * launch per call.  All calls on a device
+ * attributes) -- make it before any stream capture.  Five kernel launches
+ * per call, none of which needs all its blocks on the GPU at once: the call
+ * runs on a stream that owns a few SMs.  All calls on a device
  * share one scratch, which keeps the last call's contents (nothing in it
  * needs clearing): calls that can overlap on the GPU (different streams,
  * no ordering between them) race and must not be issued. */

@@ -15,8 +15,6 @@
 #include <cstdio>
 #include <mutex>
 
-#include <cooperative_groups.h>
-
 #include "engine.cuh"
 #include "../../include/qvti.h"
 
@@ -26,7 +24,7 @@ namespace {
 // Largest half spectrum (nz/2 + 1) * nx * ny the static scratch holds:
 // 2^19 complex values = 4 MiB (e.g. 96^3, 64 x 64 x 128, 128 x 128 x 60).
 constexpr long long kNoAllocSpectrum = 1ll << 19;
-constexpr int kNoAllocAxis = 1024;  // longest axis the static tables hold
+constexpr int kNoAllocAxis = 1024;  // longest axis
 
 // Held by every GPU that loads the library, until the process exits.
 static __device__ __align__(256) float2 g_na_scratch[kNoAllocSpectrum];
@@ -42,15 +40,21 @@ NoAllocDev g_na_dev[kMaxDevices];
 std::mutex g_na_mu;
 
 // ------------------------------------------------------------------ k_qd --
-// The whole derivative in one cooperative launch: z forward (R2C), y forward,
-// x forward - multiplier - x inverse, y inverse, z inverse (C2R), a grid
-// barrier between the passes.  The fields are small (at most 4 MiB of
-// spectrum, resident in L2), so as eight launches -- three table builds and
-// five passes -- a call was launch gaps and ramp-up: 49 us at 32 x 48 x 40, 78
-// us at 96^3; as one launch 30 and 43 us, 22 of them the passes' latencies
-// (16^3).  A pass takes tiles of P pencils, block after block; the
-// twiddles of its axis are built in FP64 in shared memory (one or two per
-// thread).
+// The derivative in five launches, one per pass: z forward (R2C), y forward, x
+// forward - multiplier - x inverse, y inverse, z inverse (C2R).  The fields are
+// small (at most 4 MiB of spectrum, resident in L2), so as eight launches --
+// three table builds and five passes -- a call was launch gaps and ramp-up: 49
+// us at 32 x 48 x 40, 78 us at 96^3 (now 31 and 41).  A pass takes tiles of P
+// pencils, block after block; the twiddles of its axis are built in FP64 in
+// shared memory.  One kernel takes the pass as an argument: five kernels fetched
+// their instructions anew at every launch (16^3 28.6 against 22.9 us, 96^3 49.2
+// against 41.4).  The launches are programmatically dependent: the next pass is
+// launched as the blocks before it end (with plain launches, 16^3 34.9 against
+// 28.6 us); releasing it earlier takes shared memory from the running one (96^3
+// 53.5 against 49.2).  Nothing needs its blocks on the GPU all at once, so the
+// call runs in a context that owns a few SMs and beside kernels that hold the
+// others; one cooperative launch with grid barriers between the passes needed
+// them all, and took 22.6 and 43.0 us.
 struct QdArgs {
     const float* in;
     float* out;
@@ -87,16 +91,14 @@ __device__ __forceinline__ float2 qd_shift(int i, int n, float h, int fwd)
     return make_float2((float)(fwd ? -t * sn : t * sn), 2 * i == n ? 0.f : (float)(i <= n / 2 ? t * cs : -t * cs));
 }
 
-__global__ void __launch_bounds__(kQdThreads) k_qd(const __grid_constant__ QdArgs a)
+__global__ void __launch_bounds__(kQdThreads) k_qd(const __grid_constant__ QdArgs a, int pass)
 {
-    namespace cg = cooperative_groups;
     extern __shared__ float4 smem4[];
     float2* sm = reinterpret_cast<float2*>(smem4);
     const int nx = a.n[0], ny = a.n[1], nz = a.n[2], P = a.P, t = threadIdx.x;
     float2 *tw = sm, *X, *A, *B;
     auto layout = [&](int ax) {
         const int n = a.n[ax], ps = n + n / 16;
-        __syncthreads();  // the previous pass's shared memory is free
         X = tw + n;
         A = X + P * ps;
         B = A + P * ps;  // used (and counted in the launch) only with more than two stages
@@ -105,12 +107,16 @@ __global__ void __launch_bounds__(kQdThreads) k_qd(const __grid_constant__ QdArg
             sincospi(-2.0 * i / n, &s, &c);
             tw[i] = make_float2((float)c, (float)s);
         }
-        __syncthreads();
         return ps;
     };
+    auto ready = [] {  // the tables, and what the passes before this one wrote
+        asm volatile("griddepcontrol.wait;" ::: "memory");
+        __syncthreads();
+    };
     // z forward: pencil q of a tile = rows (2q, 2q + 1) of the flattened (x, y)
-    {
+    if (pass == 0) {
         const int ps = layout(2), npair = nx * ny / 2, tiles = (npair + P - 1) / P;
+        ready();
         for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
             const int q0 = tile * P, qn = min(P, npair - q0);
             for (int w = t; w < P * nz; w += kQdThreads) {
@@ -130,10 +136,10 @@ __global__ void __launch_bounds__(kQdThreads) k_qd(const __grid_constant__ QdArg
             __syncthreads();
         }
     }
-    cg::this_grid().sync();
     // a y pass over the contiguous lines (kz, x)
-    auto ypass = [&](auto inv) {
+    if (pass == 1 || pass == 3) {
         const int ps = layout(1), lines = a.nkz * nx, tiles = (lines + P - 1) / P;
+        ready();
         for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
             const int l0 = tile * P, ln = min(P, lines - l0);
             float2* H = a.H + (long long)l0 * ny;
@@ -142,18 +148,17 @@ __global__ void __launch_bounds__(kQdThreads) k_qd(const __grid_constant__ QdArg
                 X[p * ps + i + (i >> 4)] = p < ln ? H[w] : make_float2(0.f, 0.f);
             }
             __syncthreads();
-            qd_lines<decltype(inv)::value != 0>(a.pl[1], tw, X, A, B, P);
+            if (pass == 3) qd_lines<true>(a.pl[1], tw, X, A, B, P);
+            else qd_lines<false>(a.pl[1], tw, X, A, B, P);
             for (int w = t; w < ln * ny; w += kQdThreads) {
                 const int p = w / ny, i = w - p * ny;
                 H[w] = X[p * ps + i + (i >> 4)];
             }
             __syncthreads();
         }
-    };
-    ypass(IntC<0>{});
-    cg::this_grid().sync();
+    }
     // x forward, |k|^pw T(k_axis) / ntp, x inverse: P consecutive y of one kz
-    {
+    if (pass == 2) {
         const int ps = layout(0), chunks = (ny + P - 1) / P, tiles = chunks * a.nkz;
         float2* tT = B + (a.pl[0].q.nst > 2 ? P * ps : 0);  // the shift over the axis it varies on
         float* tk = reinterpret_cast<float*>(tT + max(nx, P));
@@ -163,6 +168,7 @@ __global__ void __launch_bounds__(kQdThreads) k_qd(const __grid_constant__ QdArg
             tk[i] = kx * kx;
             if (a.axis == 0) tT[i] = cscale(qd_shift(i, nx, a.h[0], a.fwd), a.inv_ntp);
         }
+        ready();
         for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
             const int kz = tile / chunks, y0 = (tile - kz * chunks) * P, yn = min(P, ny - y0);
             float2* H = a.H + (long long)kz * nx * ny + y0;
@@ -194,12 +200,10 @@ __global__ void __launch_bounds__(kQdThreads) k_qd(const __grid_constant__ QdArg
             __syncthreads();
         }
     }
-    cg::this_grid().sync();
-    ypass(IntC<1>{});
-    cg::this_grid().sync();
     // z inverse (C2R)
-    {
+    if (pass == 4) {
         const int ps = layout(2), npair = nx * ny / 2, tiles = (npair + P - 1) / P;
+        ready();
         for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
             const int q0 = tile * P, qn = min(P, npair - q0);
             for (int w = t; w < P * a.nkz; w += kQdThreads) {
@@ -313,14 +317,22 @@ extern "C" int qvti_q_derivative_noalloc(const float* d_in, float* d_out, int nt
     const long long pencils = (long long)ntx * nty / 2 + nkz * ntx + nkz * nty;
     a.P = pencils < 64ll * d->sms || qd_smem(a, 8) > kMaxSmem ? 4 : 8;
     const size_t sm = qd_smem(a, a.P);
-    int per_sm = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_qd, kQdThreads, sm) != cudaSuccess || per_sm < 1)
-        return fail(QVTI_ERR_CUDA);
-    const long long tiles = (std::max({(long long)ntx * nty / 2, nkz * ntx, nkz * nty}) + a.P - 1) / a.P;
-    const int blocks = (int)std::min<long long>(tiles, (long long)std::min(per_sm, 4) * d->sms);
-    void* args[] = {&a};
-    cudaLaunchCooperativeKernel((const void*)k_qd, dim3(blocks), dim3(kQdThreads), args, sm,
-                                static_cast<cudaStream_t>(stream));
+    const long long pairs = (long long)ntx * nty / 2, chunks = nkz * ((nty + a.P - 1) / a.P);
+    const long long tiles[5] = {(pairs + a.P - 1) / a.P, (nkz * ntx + a.P - 1) / a.P, chunks, (nkz * ntx + a.P - 1) / a.P,
+                                (pairs + a.P - 1) / a.P};
+    cudaLaunchAttribute at{};
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    for (int p = 0; p < 5; ++p) {
+        cudaLaunchConfig_t c{};
+        c.gridDim = dim3((unsigned)std::min<long long>(tiles[p], 4ll * d->sms));
+        c.blockDim = dim3(kQdThreads);
+        c.dynamicSmemBytes = sm;
+        c.stream = static_cast<cudaStream_t>(stream);
+        c.attrs = &at;
+        c.numAttrs = p ? 1 : 0;  // the first pass waits for what the caller queued
+        if (cudaLaunchKernelEx(&c, k_qd, a, p) != cudaSuccess) break;
+    }
     const cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) {
         fprintf(stderr, "qvti_q_derivative_noalloc: launch: %s\n", cudaGetErrorString(e));
