@@ -70,8 +70,7 @@ bool make_plan(int n, FftPlan* p)
 // its real part -- the Hermitian part of the multiplier, which is what the
 // real part of the reference's C2C output sees; C-PML a, b (cu:213-309,
 // velp_max forced to 5000, R = 1e-2, pi = 3.1415926) and their half-point
-// averages 0.5 (v[i] + v[i+1]); with a == nullptr the C-PML outputs are not
-// written (a, b, ah, bh may all be null then).
+// averages 0.5 (v[i] + v[i+1]).
 __global__ void k_axis_tables(int n, double d, double f0, int pml, float2* tw, float* kmag, float2* F, float2* B,
                               float* a, float* b, float* ah, float* bh)
 {
@@ -90,7 +89,6 @@ __global__ void k_axis_tables(int n, double d, double f0, int pml, float2* tw, f
         if (2 * i == n) { fi = 0.0; bi = 0.0; }
         F[i] = make_float2((float)fr, (float)fi);
         B[i] = make_float2((float)br, (float)bi);
-        if (!a) continue;  // no C-PML profiles wanted (spectral stages only)
         auto prof = [&](int j, double* av, double* bv) {
             const double alpha_max = pi_ref * f0;
             const double om_max = 4.0 * 5000.0 * log(1.0 / (double)1e-2f) / (2.0 * pml * d);
@@ -153,12 +151,6 @@ __global__ void k_finite3(long long n4, const float4* a, const float4* b, const 
 }  // namespace
 
 bool make_fft_plan(int n, FftPlan* p) { return make_plan(n, p); }
-
-void launch_axis_tables(int n, double d, double f0, int pml, float2* tw, float* kmag, float2* F, float2* B,
-                        float* a, float* b, float* ah, float* bh, cudaStream_t st)
-{
-    k_axis_tables<<<4, 256, 0, st>>>(n, d, f0, pml, tw, kmag, F, B, a, b, ah, bh);
-}
 
 struct Sim {
     qvti_config cfg{};

@@ -175,10 +175,8 @@ int configure_device(int dev);
 // return it.
 int fail(int code);
 
-// Radix plan of a transform length; FP64 build of one axis's 1D tables.
+// Radix plan of a transform length.
 bool make_fft_plan(int n, FftPlan* p);
-void launch_axis_tables(int n, double d, double f0, int pml, float2* tw, float* kmag, float2* F, float2* B,
-                        float* a, float* b, float* ah, float* bh, cudaStream_t st);
 
 // Tensor-core form (tc_dft.cu): 256-point y transforms on tcgen05.
 bool tc_cy_available(const KP& k);
