@@ -28,6 +28,7 @@ int fail(int code)
 // entry point uses it, with that device current.
 namespace {
 PerDeviceOnce<kMaxDevices> g_configured;
+PerDeviceOnce<kMaxDevices> g_lengths[3][1024 / 2 + 1];  // by axis and half the length
 std::atomic<long long> g_sims_created{0};
 }  // namespace
 
@@ -267,7 +268,7 @@ int slab_arrays(const KP& k, float** out, size_t* len)
 }
 constexpr int kNumSlab = 9 + 8 + 8 + 6 + 6;
 
-// Steps per multi-step graph: 16 steps are 128 kernel nodes, and a chunk of
+// Steps per multi-step graph: 16 steps are 160 kernel nodes, and a chunk of
 // the scheduler (32 steps) is two launches.
 constexpr int kGraphSteps = 16;
 
@@ -321,6 +322,12 @@ extern "C" int qvti_create(const qvti_config* cfg, qvti_sim** out)
 
     QV_CUDA(cudaSetDevice(cfg->device));
     if (configure_device(cfg->device)) return fail(QVTI_ERR_CUDA);
+    // the compiled kernels of this grid's lengths only: loading those of every
+    // length made the first simulation of a process wait 0.2 s
+    const int len[3] = {nx, ny, nz};
+    for (int a = 0; a < 3; ++a)
+        if (g_lengths[a][len[a] / 2].run(cfg->device, [&] { return configure_length(a, len[a]); }))
+            return fail(QVTI_ERR_CUDA);
 
     Sim* s = new (std::nothrow) qvti_sim();
     if (!s) return fail(QVTI_ERR_OOM);

@@ -168,7 +168,10 @@ void launch_coef_build(const KP& kp, const float* velp, const float* vels, const
                        const float* gp, const float* gs, const float* eps, const float* delta, int vti,
                        float w0, int lossless, float* const* coef_out, cudaStream_t st);
 void launch_mu_rinv(const KP& kp, const float* rho, const float* const* sset, cudaStream_t st);
-int configure_kernels();   // raise dynamic shared-memory limits, returns cudaError_t
+// Load kernels and raise their dynamic shared-memory limits: the runtime-length
+// ones, and the compiled ones that transform axis 0..2 at length n.  cudaError_t.
+int configure_kernels();
+int configure_length(int axis, int n);
 // configure_kernels() once per device (the device must be current); 0 = ok.
 int configure_device(int dev);
 // Record `code` as the calling thread's last error (qvti_last_error) and

@@ -701,7 +701,7 @@ __global__ void __launch_bounds__(kThreads) k_dzr(KP k, int P)
 }  // namespace
 
 QVTI_DECLARE_PARTS(bool, st_launch, const KP& k, int P, cudaStream_t st);
-QVTI_DECLARE_PARTS(bool, st_configure, SmemLimit& lim);
+QVTI_DECLARE_PARTS(bool, st_configure, SmemLimit& lim, int n);
 
 template <>
 bool st_launch<QVTI_PART>(const KP& k, int P, cudaStream_t st)
@@ -729,22 +729,20 @@ bool st_launch<QVTI_PART>(const KP& k, int P, cudaStream_t st)
     });
 }
 template <>
-bool st_configure<QVTI_PART>(SmemLimit& lim)
+bool st_configure<QVTI_PART>(SmemLimit& lim, int n)
 {
-    for (int n : kMyLengths)
-        dispatch_len(n, [&](auto NN) {
-            constexpr int N = decltype(NN)::value;
-            if constexpr (N >= kMinLong) {
-                lim.set((const void*)k_st<N, 9, 1>);
-                lim.set((const void*)k_st<N, 6, 1>);
-                if constexpr (st_eight_rows(N)) {
-                    lim.set((const void*)k_st<N, 9, 2>);
-                    lim.set((const void*)k_st<N, 6, 2>);
-                }
-                lim.set((const void*)k_dz<N>);
+    return dispatch_len(n, [&](auto NN) {
+        constexpr int N = decltype(NN)::value;
+        if constexpr (N >= kMinLong) {
+            lim.set((const void*)k_st<N, 9, 1>);
+            lim.set((const void*)k_st<N, 6, 1>);
+            if constexpr (st_eight_rows(N)) {
+                lim.set((const void*)k_st<N, 9, 2>);
+                lim.set((const void*)k_st<N, 6, 2>);
             }
-        });
-    return false;
+            lim.set((const void*)k_dz<N>);
+        }
+    });
 }
 
 #if QVTI_PART == 0
@@ -770,12 +768,15 @@ void launch_sigma(const KP& k, int P, bool rt, cudaStream_t st)
     k_dzr<<<dim3(tiles, k.nx, 3), rt_threads(k.pz, P / 2), sm, st>>>(k, P);
 }
 
-cudaError_t configure_sigma()
+cudaError_t configure_sigma(int axis, int n)
 {
     SmemLimit lim;
-    lim.set((const void*)k_sigma);
-    lim.set((const void*)k_dzr);
-    (void)QVTI_CALL_PARTS(st_configure, lim);
+    if (axis < 0) {
+        lim.set((const void*)k_sigma);
+        lim.set((const void*)k_dzr);
+    } else if (axis == 2) {
+        (void)QVTI_CALL_PARTS(st_configure, lim, n);
+    }
     return lim.e;
 }
 #endif  // QVTI_PART == 0

@@ -468,7 +468,7 @@ QVTI_DECLARE_PARTS(bool, fz_launch, const KP& k, int P, int ncomp, cudaStream_t 
 QVTI_DECLARE_PARTS(bool, cy_launch, const KP& k, bool inv, dim3 grid, long long line0, long long line_end,
                    cudaStream_t st);
 QVTI_DECLARE_PARTS(bool, mx_launch, const KP& k, int P, int kz0, int nb, cudaStream_t st);
-QVTI_DECLARE_PARTS(bool, sp_configure, SmemLimit& lim);
+QVTI_DECLARE_PARTS(bool, sp_configure, SmemLimit& lim, int axis, int n);
 
 template <>
 bool fz_launch<QVTI_PART>(const KP& k, int P, int ncomp, cudaStream_t st)
@@ -497,17 +497,18 @@ bool mx_launch<QVTI_PART>(const KP& k, int P, int kz0, int nb, cudaStream_t st)
     });
 }
 template <>
-bool sp_configure<QVTI_PART>(SmemLimit& lim)
+bool sp_configure<QVTI_PART>(SmemLimit& lim, int axis, int n)
 {
-    for (int n : kMyLengths)
-        dispatch_len(n, [&](auto NN) {
-            constexpr int N = decltype(NN)::value;
-            lim.set((const void*)k_fp<N>);
+    return dispatch_len(n, [&](auto NN) {
+        constexpr int N = decltype(NN)::value;
+        if (axis == 2) lim.set((const void*)k_fp<N>);
+        if (axis == 1) {
             lim.set((const void*)k_cp<N, false>);
             lim.set((const void*)k_cp<N, true>);
-            if constexpr (N >= kMinLong) lim.set((const void*)k_mp<N>);
-        });
-    return false;
+        }
+        if constexpr (N >= kMinLong)
+            if (axis == 0) lim.set((const void*)k_mp<N>);
+    });
 }
 
 #if QVTI_PART == 0
@@ -550,14 +551,17 @@ void launch_mx(const KP& k, int P, bool rt, int kz0, int nb, cudaStream_t st)
     else (void)QVTI_CALL_PARTS(mx_launch, k, P, kz0, nb, st);
 }
 
-cudaError_t configure_spectral()
+cudaError_t configure_spectral(int axis, int n)
 {
     SmemLimit lim;
-    lim.set((const void*)k_fz);
-    lim.set((const void*)k_cy<false>);
-    lim.set((const void*)k_cy<true>);
-    lim.set((const void*)k_mx);
-    (void)QVTI_CALL_PARTS(sp_configure, lim);
+    if (axis < 0) {
+        lim.set((const void*)k_fz);
+        lim.set((const void*)k_cy<false>);
+        lim.set((const void*)k_cy<true>);
+        lim.set((const void*)k_mx);
+    } else {
+        (void)QVTI_CALL_PARTS(sp_configure, lim, axis, n);
+    }
     return lim.e;
 }
 #endif  // QVTI_PART == 0

@@ -607,7 +607,7 @@ __global__ void __launch_bounds__(dv_threads(N, PP), dv_blocks(N, PP)) k_dv(KP k
 }  // namespace
 
 QVTI_DECLARE_PARTS(bool, dv_launch, const KP& k, int ax, int P, cudaStream_t st);
-QVTI_DECLARE_PARTS(bool, dv_configure, SmemLimit& lim);
+QVTI_DECLARE_PARTS(bool, dv_configure, SmemLimit& lim, int ax, int n);
 
 template <>
 bool dv_launch<QVTI_PART>(const KP& k, int ax, int P, cudaStream_t st)
@@ -629,20 +629,21 @@ bool dv_launch<QVTI_PART>(const KP& k, int ax, int P, cudaStream_t st)
     });
 }
 template <>
-bool dv_configure<QVTI_PART>(SmemLimit& lim)
+bool dv_configure<QVTI_PART>(SmemLimit& lim, int ax, int n)
 {
-    for (int n : kMyLengths)
-        dispatch_len(n, [&](auto NN) {
-            constexpr int N = decltype(NN)::value;
-            auto set = [&](auto AX) {
-                constexpr int ax = decltype(AX)::value;
-                lim.set((const void*)k_dv<N, 8, ax>);
-                lim.set((const void*)k_dv<N, 16, ax>);
-            };
+    return dispatch_len(n, [&](auto NN) {
+        constexpr int N = decltype(NN)::value;
+        auto set = [&](auto AX) {
+            constexpr int ax_ = decltype(AX)::value;
+            lim.set((const void*)k_dv<N, 8, ax_>);
+            lim.set((const void*)k_dv<N, 16, ax_>);
+        };
+        if (ax) {
             set(IntC<1>{});
+        } else {
             if constexpr (N >= kMinLong) set(IntC<0>{});
-        });
-    return false;
+        }
+    });
 }
 
 #if QVTI_PART == 0
@@ -660,12 +661,15 @@ void launch_vx(const KP& k, int P, bool rt, cudaStream_t st)
     else (void)QVTI_CALL_PARTS(dv_launch, k, 0, P, st);
 }
 
-cudaError_t configure_velocity()
+cudaError_t configure_velocity(int axis, int n)
 {
     SmemLimit lim;
-    lim.set((const void*)k_vy);
-    lim.set((const void*)k_vx);
-    (void)QVTI_CALL_PARTS(dv_configure, lim);
+    if (axis < 0) {
+        lim.set((const void*)k_vy);
+        lim.set((const void*)k_vx);
+    } else if (axis < 2) {
+        (void)QVTI_CALL_PARTS(dv_configure, lim, axis, n);
+    }
     return lim.e;
 }
 #endif  // QVTI_PART == 0

@@ -140,10 +140,12 @@ size_t smem_fz(const KP& k, int P, bool rt);
 size_t smem_cy(const KP& k, int L, bool ydv, bool rt);
 size_t smem_mx(const KP& k, int P, bool rt);
 size_t smem_sigma(const KP& k, int P, bool rt);
-// Raise the dynamic shared-memory limit of every instantiation; cudaError_t.
-cudaError_t configure_velocity();
-cudaError_t configure_spectral();
-cudaError_t configure_sigma();
+// Load kernels and raise their dynamic shared-memory limit: the runtime forms
+// (axis < 0), or the compiled ones that transform axis 0 (x), 1 (y) or 2 (z) at
+// length n; cudaError_t.
+cudaError_t configure_velocity(int axis, int n);
+cudaError_t configure_spectral(int axis, int n);
+cudaError_t configure_sigma(int axis, int n);
 
 // cudaFuncSetAttribute over kernels, keeping the last error.
 struct SmemLimit {

@@ -319,11 +319,19 @@ int configure_kernels()
     lim.set((const void*)k_deriv1d);
     lim.set((const void*)kq_mx);
     lim.set((const void*)kq_iz);
-    for (cudaError_t r : {configure_velocity(), configure_spectral(), configure_sigma()})
+    for (cudaError_t r : {configure_velocity(-1, 0), configure_spectral(-1, 0), configure_sigma(-1, 0)})
         if (r != cudaSuccess) lim.e = r;
     const int et = configure_tc_kernels();
     if (et) lim.e = (cudaError_t)et;
     return (int)lim.e;
+}
+
+int configure_length(int axis, int n)
+{
+    cudaError_t e = cudaSuccess;
+    for (cudaError_t r : {configure_velocity(axis, n), configure_spectral(axis, n), configure_sigma(axis, n)})
+        if (r != cudaSuccess) e = r;
+    return (int)e;
 }
 
 const char* const kStepKernelNames[kStepKernels] = {"k_vy",  "k_vx",     "k_fz",    "k_cy_fwd",
