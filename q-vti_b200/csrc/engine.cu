@@ -956,8 +956,8 @@ static void kernel_bytes(const qvti_sim* s, double* b)
     b[4] = 3 * S + qvti::kNumGxy * S;                                      // k_mx
     b[5] = qvti::kNumGxy * 2 * S;                                          // k_cy_inv
     // k_sigma: 27 half spectra (21 G, 3 H, 3 Yv), 6 stresses and 6 loss potentials read+written,
-    // model + MU, 3 R written, C-PML variables in their slabs
-    b[6] = qvti::kNumG * S + 12 * F + 12 * F + model + 5 * F + 3 * F + 3 * 8 * cz +
+    // model + MU, 3 stresses read again by k_dz, 3 R written, C-PML variables in their slabs
+    b[6] = qvti::kNumG * S + 12 * F + 12 * F + model + 5 * F + 3 * F + 3 * F + 3 * 8 * cz +
            (48 + 16 + 16) * cx + (48 + 16 + 16) * cy + (32 + 16 + 16) * cz;
     b[7] = s->rn * (3 * 4.0 * 2 + 8.0);                                    // k_rec
 }

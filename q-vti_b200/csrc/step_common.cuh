@@ -44,9 +44,10 @@ __device__ __forceinline__ void fft_rt(const FftPlan& pl, const float2* tw, floa
 }
 
 // Transform lengths with a compile-time path: the 5-smooth lengths the
-// batching and serving workloads draw between 96 and 384, 512, and the other
-// even 7-smooth lengths from 24 up to the serving range; a kernel takes it
-// when its transform length is listed, otherwise the runtime path.  The
+// batching and serving workloads draw between 96 and 384, 512, and most other
+// even 7-smooth lengths from 24 to 252 (of those above, 280, 294, 336, 350 and
+// 378 are not listed); a kernel takes it when its transform length is listed,
+// otherwise the runtime path.  The
 // shortest lengths, below 36, come for k_vy, k_fz and k_cy only: the tile tests
 // run the x kernels' runtime form at 32, and the stress update of so short a z
 // axis is faster in its runtime form with 16 rows per block (32^3: 26 us) than
@@ -122,8 +123,8 @@ inline int cdiv(int a, int b) { return (a + b - 1) / b; }
 __host__ __device__ constexpr int mp_rows(int n) { return radix_seq(n).nst > 2 ? 8 : 16; }
 
 // Lengths whose compiled stress kernels also come with eight rows: those of two
-// stages (three have up to 64 butterflies a pencil, and eighteen pencils would
-// pass the threads of a block).
+// stages (at three, 18 .. 40 threads a pencil pair, eighteen pairs are a block of
+// up to 720 threads, and its exchange most of an SM's shared memory).
 __host__ __device__ constexpr bool st_eight_rows(int n) { return radix_seq(n).nst == 2; }
 
 // One kernel of the step: tile `P`, rt = the runtime-length kernel.

@@ -347,8 +347,9 @@ void launch_step(const KP& k, cudaStream_t st, StepProfile* prof)
             prof->kind[prof->n++] = kind;
         }
     };
-    // the compile-time path of a kernel fixes its tile: 16 z rows (k_vy,
-    // k_vx), 16 y rows (k_fz, k_mx), 8 lines (k_cy), kSigmaRows y rows
+    // the compile-time path of a kernel fixes its tile: 16 or 32 z (k_vy, k_vx;
+    // dv_tile), 16 y rows (k_fz), 16 or 8 (k_mx; mp_rows), 8 lines (k_cy), 4 or
+    // 8 y rows (k_sigma; st_rows)
     const StepTiles T = step_tiles(k);
     mark(-1);
     launch_vy(k, T.vy, T.rt[0], st);
