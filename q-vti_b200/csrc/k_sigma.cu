@@ -34,11 +34,10 @@ __device__ __forceinline__ void prefetch_l2(const void* p, unsigned bytes)
 // 32 neighbouring lanes (a second load otherwise: 2.65 against 2.2 ms).  With
 // eight rows (Q = 2) the two row quads of a butterfly are neighbouring lanes and
 // read 64 bytes of a line between them: a warp's load touches 16 lines instead
-// of 32 (shear 0.68 against 0.78 ms at 256^3, the whole update 1.40 against 1.52).
+// of 32 (shear 0.68 against 0.78 ms at 256^3).
 constexpr int st_threads(int n, int nf, int q) { return warps_up(nf * q * pair_tasks(n)); }
 constexpr size_t st_smem(int n, int nf, int q) { return 16 * ((size_t)nf * q * pair_slots_q(n, q) + tw_rows_size(n)); }
-// Blocks per SM the registers are sized for (256 points, normal stresses: two
-// blocks of nine warps at 96 registers 0.536 ms, one at 158 0.577).
+// Blocks per SM the registers are sized for: 16 to 20 warps.
 constexpr int st_blocks(int n, int nf, int q)
 {
     const int warps = st_threads(n, nf, q) / 32, m = (int)(220 * 1024 / (st_smem(n, nf, q) + 2048));
@@ -46,6 +45,17 @@ constexpr int st_blocks(int n, int nf, int q)
     if (b < 1) b = 1;
     return b < m ? b : m < 1 ? 1 : m;
 }
+// Whether stage 0 gets its mirror points by shuffle.
+constexpr bool st_shuffles(int n, int q)
+{
+    const int lanes = pair_tasks(n) * q;
+    return pair_rad(n, 0) % 2 == 0 && pair_k(n, 0) == 1 && (lanes == 8 || lanes == 16 || lanes == 32);
+}
+// Rows of a normal-stress block in quads where the shear blocks take q: one where
+// four rows shuffle (nine fields of two quads leave 96 registers a thread at 256
+// points, and spills: 1.48 against 1.40 ms for the whole update at 256^3, 0.220
+// against 0.208 at 128^3), else the shear blocks' (98 points: 0.217 against 0.235).
+constexpr int st_normal_q(int n, int q) { return st_shuffles(n, 1) ? 1 : q; }
 // Whether a compiled z length takes sxy's two terms one after the other (see
 // stress_pair): the 5-smooth lengths from 96, 64 and 512.
 constexpr bool st_halves(int n)
@@ -74,38 +84,35 @@ __device__ __forceinline__ void put2(float* p, int n, bool second, f2 v)
 // Constant-Q set of one modulus for two rows from its effective velocity
 // c = v cos(pi g/2) (cuviscoelas_3D.cu:195-205): eta1 = -rho c g w0, eta2 =
 // rho c^2, eta3 = rho c^3 g / w0, tau1 = rho c g pi, tau2 = rho c^2 g^2 pi / w0.
-// c is built in FP64 at setup; the products are rebuilt here in FP32.  The last
-// factor of each comes apart (o = m f), for sums that round the product only
-// once.
-struct QSet {
-    f2 m[5], f[5], o[5];
+// c is built in FP64 at setup; the products are rebuilt here in FP32, one of the
+// five at a time.  The last factor comes apart (o = m f), for sums that round the
+// product only once.
+struct Mod {
+    f2 rc, c, g;
 };
-__device__ __forceinline__ void qset2(QSet& s, f2 rho, f2 c, f2 g, float w0, float inv_w0)
+struct Coef {
+    f2 m, f, o;
+};
+__device__ __forceinline__ Coef coef(const Mod& s, int j, float w0, float inv_w0)
 {
     const float pi = 3.1415926f;
-    const f2 rc = rho * c, rc2 = rc * c;
-    s.m[0] = neg_(rc) * g;          s.f[0] = bc(w0);
-    s.m[1] = rc;                    s.f[1] = c;
-    s.m[2] = rc2 * c * g;           s.f[2] = bc(inv_w0);
-    s.m[3] = rc * g;                s.f[3] = bc(pi);
-    s.m[4] = rc2 * g * g * bc(pi);  s.f[4] = bc(inv_w0);
-#pragma unroll
-    for (int j = 0; j < 5; ++j) s.o[j] = s.m[j] * s.f[j];
+    Coef r;
+    if (j == 0) { r.m = neg_(s.rc) * s.g; r.f = bc(w0); }
+    else if (j == 1) { r.m = s.rc; r.f = s.c; }
+    else if (j == 2) { r.m = s.rc * s.c * s.c * s.g; r.f = bc(inv_w0); }
+    else if (j == 3) { r.m = s.rc * s.g; r.f = bc(pi); }
+    else { r.m = s.rc * s.c * s.g * s.g * bc(pi); r.f = bc(inv_w0); }
+    r.o = r.m * r.f;
+    return r;
 }
 // a13 - 2 a55 of two sets, the product of a13 (but that of eta2, which eta3
 // shares) not rounded by itself
-__device__ __forceinline__ f2 less13(const QSet& a, const QSet& s5, int j)
+__device__ __forceinline__ f2 less13(const Coef& a, const Coef& s5, int j)
 {
-    return j == 1 ? fma_(bc(-2.f), s5.o[j], a.o[j]) : fma_(a.m[j], a.f[j], s5.o[j] * bc(-2.f));
+    return j == 1 ? fma_(bc(-2.f), s5.o, a.o) : fma_(a.m, a.f, s5.o * bc(-2.f));
 }
-__device__ __forceinline__ f2 dot3(const f2* a, f2 x, f2 y, f2 z, int v = 0)
-{
-    return v ? fma_(a[2], z, fma_(a[1], y, a[0] * x)) : fma_(a[2], z, fma_(a[0], x, a[1] * y));
-}
-__device__ __forceinline__ f2 dot2(const f2* a, f2 x, f2 y, int v = 0)
-{
-    return v ? fma_(a[4], y, a[3] * x) : fma_(a[3], x, a[4] * y);
-}
+__device__ __forceinline__ f2 dot3(const f2* a, f2 x, f2 y, f2 z) { return fma_(a[2], z, fma_(a[0], x, a[1] * y)); }
+__device__ __forceinline__ f2 dot2(const f2* a, f2 x, f2 y) { return fma_(a[3], x, a[4] * y); }
 
 // One C-PML term of a row pair: the slab's memory variable and loss potential
 // (second row n further on), loaded, then advanced by the term d and its new
@@ -271,38 +278,46 @@ __device__ __forceinline__ void stress_pair(const KP& k, int n, int grp, int x, 
             zload(6, k.phn[6], k.qn[6]);
             zload(7, k.phn[7], k.qn[7]);
         }
-        f2 a11[5], a33[5], a13[5], a12[5];
+        // the sets one coefficient at a time, each into the sums of all terms:
+        // their products in the order 1, 0, 2 (d33z: 0, 1, 2) and 4, 3
+        f2 d11x, d12x, d13x, d12y, d11y, d13y, d13z, d33z, q11x, q12x, q13x, q12y, q11y, q13y, q13z, q33z;
         {
-            QSet s5, q;
-            qset2(s5, rho, cs, gs, w0, inv_w0);
-            qset2(q, rho, c33, gp, w0, inv_w0);
-#pragma unroll
-            for (int j = 0; j < 5; ++j) {
-                a33[j] = a11[j] = q.o[j];
-                a12[j] = fma_(bc(-2.f), s5.o[j], q.o[j]);
-                a13[j] = less13(q, s5, j);
-            }
-            if (aniso) {
-                qset2(q, rho, c11, gp, w0, inv_w0);
-#pragma unroll
-                for (int j = 0; j < 5; ++j) {
-                    a11[j] = q.o[j];
-                    a12[j] = fma_(bc(-2.f), s5.o[j], q.o[j]);
-                }
-                qset2(q, rho, c13, gp, w0, inv_w0);
-#pragma unroll
-                for (int j = 0; j < 5; ++j) a13[j] = less13(q, s5, j);
-            }
+            const Mod m33{rho * c33, c33, gp}, m11{rho * c11, c11, gp}, m13{rho * c13, c13, gp}, m5{rho * cs, cs, gs};
+            auto sets = [&](int j, f2& a11, f2& a12, f2& a13, f2& a33) {
+                const Coef s5 = coef(m5, j, w0, inv_w0), k33 = coef(m33, j, w0, inv_w0);
+                const Coef k11 = aniso ? coef(m11, j, w0, inv_w0) : k33, k13 = aniso ? coef(m13, j, w0, inv_w0) : k33;
+                a33 = k33.o;
+                a11 = k11.o;
+                a12 = fma_(bc(-2.f), s5.o, a11);
+                a13 = less13(k13, s5, j);
+            };
+            f2 a11, a12, a13, a33;
+            f2 X = sv(1), Y = sv(4), Z = sv(7);
+            sets(1, a11, a12, a13, a33);
+            d11x = a11 * X; d12x = a12 * X; d13x = a13 * X;
+            d12y = a12 * Y; d11y = a11 * Y; d13y = a13 * Y;
+            d13z = a13 * Z;
+            const f2 a33_1 = a33;
+            sets(4, a11, a12, a13, a33);
+            q11x = a11 * X; q12x = a12 * X; q13x = a13 * X;
+            q12y = a12 * Y; q11y = a11 * Y; q13y = a13 * Y;
+            q13z = a13 * Z; q33z = a33 * Z;
+            const f2 Z1 = Z;
+            X = sv(0); Y = sv(3); Z = sv(6);
+            sets(0, a11, a12, a13, a33);
+            d11x = fma_(a11, X, d11x); d12x = fma_(a12, X, d12x); d13x = fma_(a13, X, d13x);
+            d12y = fma_(a12, Y, d12y); d11y = fma_(a11, Y, d11y); d13y = fma_(a13, Y, d13y);
+            d13z = fma_(a13, Z, d13z); d33z = fma_(a33_1, Z1, a33 * Z);
+            sets(3, a11, a12, a13, a33);
+            q11x = fma_(a11, X, q11x); q12x = fma_(a12, X, q12x); q13x = fma_(a13, X, q13x);
+            q12y = fma_(a12, Y, q12y); q11y = fma_(a11, Y, q11y); q13y = fma_(a13, Y, q13y);
+            q13z = fma_(a13, Z, q13z); q33z = fma_(a33, Z, q33z);
+            X = sv(2); Y = sv(5); Z = sv(8);
+            sets(2, a11, a12, a13, a33);
+            d11x = fma_(a11, X, d11x); d12x = fma_(a12, X, d12x); d13x = fma_(a13, X, d13x);
+            d12y = fma_(a12, Y, d12y); d11y = fma_(a11, Y, d11y); d13y = fma_(a13, Y, d13y);
+            d13z = fma_(a13, Z, d13z); d33z = fma_(a33, Z, d33z);
         }
-        f2 X = sv(0), Y = sv(1), Z = sv(2);
-        const f2 d11x = dot3(a11, X, Y, Z), d12x = dot3(a12, X, Y, Z), d13x = dot3(a13, X, Y, Z);
-        const f2 q11x = dot2(a11, X, Y), q12x = dot2(a12, X, Y), q13x = dot2(a13, X, Y);
-        X = sv(3); Y = sv(4); Z = sv(5);
-        const f2 d12y = dot3(a12, X, Y, Z), d11y = dot3(a11, X, Y, Z), d13y = dot3(a13, X, Y, Z);
-        const f2 q12y = dot2(a12, X, Y), q11y = dot2(a11, X, Y), q13y = dot2(a13, X, Y);
-        X = sv(6); Y = sv(7); Z = sv(8);
-        const f2 d13z = dot3(a13, X, Y, Z), d33z = dot3(a33, X, Y, Z, 1);
-        const f2 q13z = dot2(a13, X, Y), q33z = dot2(a33, X, Y);
         // loss: sum_terms tau-coefficient x (S - S_prev)/dt = (Q - Q_prev)/dt
         const f2 Qxx = q11x + q12y + q13z, Qyy = q12x + q11y + q13z, Qzz = q13x + q13y + q33z;
         f2 txx = fma_(Qxx - qx, inv_dt, d11x + d12y + d13z);
@@ -387,8 +402,8 @@ __global__ void __launch_bounds__(st_threads(N, NF, Q), st_blocks(N, NF, Q)) k_s
 {
     using F = PairFFT<N, NF * Q, false, Q>;
     constexpr int NT = st_threads(N, NF, Q), R0 = F::R0, NR0 = N / R0, ROWS = 4 * Q, LANES = F::T * Q;
+    constexpr bool SHFL = st_shuffles(N, Q);
     static_assert(NT <= 1024, "threads of a block");
-    constexpr bool SHFL = R0 % 2 == 0 && F::K0 == 1 && (LANES == 8 || LANES == 16 || LANES == 32);
     extern __shared__ float4 smem4[];
     f2* buf = reinterpret_cast<f2*>(smem4);
     float4* tw = smem4 + F::PLANE;
@@ -709,11 +724,10 @@ bool st_launch<QVTI_PART>(const KP& k, int P, cudaStream_t st)
     return dispatch_len(k.nz, [&](auto NN) {
         constexpr int N = decltype(NN)::value;
         if constexpr (N >= kMinLong) {
-            const int tiles = cdiv(k.ny, P);
             auto go = [&](auto QQ) {
-                constexpr int q = decltype(QQ)::value;
-                k_st<N, 9, q><<<dim3(tiles, k.nx), st_threads(N, 9, q), st_smem(N, 9, q), st>>>(k);
-                k_st<N, 6, q><<<dim3(3 * tiles, k.nx), st_threads(N, 6, q), st_smem(N, 6, q), st>>>(k);
+                constexpr int q = decltype(QQ)::value, q9 = st_normal_q(N, q);
+                k_st<N, 9, q9><<<dim3(cdiv(k.ny, 4 * q9), k.nx), st_threads(N, 9, q9), st_smem(N, 9, q9), st>>>(k);
+                k_st<N, 6, q><<<dim3(3 * cdiv(k.ny, P), k.nx), st_threads(N, 6, q), st_smem(N, 6, q), st>>>(k);
             };
             if constexpr (st_eight_rows(N)) {
                 if (P == 8) {
@@ -737,7 +751,7 @@ bool st_configure<QVTI_PART>(SmemLimit& lim, int n)
             lim.set((const void*)k_st<N, 9, 1>);
             lim.set((const void*)k_st<N, 6, 1>);
             if constexpr (st_eight_rows(N)) {
-                lim.set((const void*)k_st<N, 9, 2>);
+                lim.set((const void*)k_st<N, 9, st_normal_q(N, 2)>);
                 lim.set((const void*)k_st<N, 6, 2>);
             }
             lim.set((const void*)k_dz<N>);
