@@ -50,8 +50,9 @@ __device__ __forceinline__ void fft_rt(const FftPlan& pl, const float2* tw, floa
 // otherwise the runtime path.  The
 // shortest lengths, below 36, come for k_vy, k_fz and k_cy only: the tile tests
 // run the x kernels' runtime form at 32, and the stress update of so short a z
-// axis is faster in its runtime form with 16 rows per block (32^3: 26 us) than
-// as the compiled kernels' three launches (28).
+// axis was faster in its runtime form with 16 rows per block (32^3: 26 us) than
+// as the compiled kernels' three launches (28) when both ran 32 as 8 4; as 16 2 the
+// runtime form takes 31.
 constexpr int kMinLong = 36;
 //
 // The lengths are split into QVTI_PARTS lists: each unit of compiled kernels is

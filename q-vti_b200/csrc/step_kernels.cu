@@ -276,8 +276,8 @@ bool ct_length(int n)
 //
 // The compiled velocity kernels take 32 z (whole 128-byte rows: 16 z left
 // half of every L1 line it fetched unused and measured 0.21 against 0.15 ms
-// for k_vy, 0.34 against 0.22 for k_vx at 256^3) unless that leaves fewer than
-// two blocks per SM.
+// for k_vy, 0.34 against 0.22 for k_vx at 256^3, with the epilogue on registers)
+// unless that leaves fewer than two blocks per SM.
 int dv_tile(int nz, int lines) { return 3ll * cdiv(nz, 64) * lines >= 2 * 148 ? 32 : 16; }
 // The compiled stress kernels take eight rows (half-line accesses, see k_st)
 // unless that leaves fewer than four blocks per SM.
