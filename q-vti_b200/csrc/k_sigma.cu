@@ -57,7 +57,8 @@ constexpr bool st_shuffles(int n, int q)
 // against 0.208 at 128^3), else the shear blocks' (98 points: 0.217 against 0.235).
 constexpr int st_normal_q(int n, int q) { return st_shuffles(n, 1) ? 1 : q; }
 // Whether a compiled z length takes sxy's two terms one after the other (see
-// stress_pair): the 5-smooth lengths from 96, 64 and 512.
+// stress_pair): 64 and the 5-smooth lengths from 96, whose scalar kernel did (the
+// other lengths had the runtime one).
 constexpr bool st_halves(int n)
 {
     if (n < 96) return n == 64;
@@ -445,6 +446,7 @@ __global__ void __launch_bounds__(st_threads(N, NF, Q), st_blocks(N, NF, Q)) k_s
             a[0] = make_float2(u.x, u.y); a[1] = make_float2(u.z, u.w);
             a[2] = make_float2(w.x, w.y); a[3] = make_float2(w.z, w.w);
             if (gz) {
+                // (rounded as the scalar kernels of these lengths did)
                 const float2 m = cscale(M[kk], inv_nz);
 #pragma unroll
                 for (int q = 0; q < 4; ++q) a[q] = st_halves(N) ? cmul_m(a[q], m) : cmul(a[q], m);
